@@ -136,6 +136,13 @@ int build_device_symbolic(orbit_symbolic_s* h) {
     ORBIT_TRY(upload(A, &q.nchunk_fwdT, Q.nchunk_fwdT));
     ORBIT_TRY(upload(A, &q.nchunk_bwdT, Q.nchunk_bwdT));
   }
+  for (int k = 0; k < kNumSched && S.max_sub_front == 0; ++k)
+    for (int v = 0; v < 3; ++v) {
+      const FlowSched& Q = v < 2 ? S.staged[k][v] : S.columns[k];
+      DevSym::Flow& q = v < 2 ? d.staged[k][v] : d.columns[k];
+      ORBIT_TRY(upload(A, &q.recs, Q.recs));
+      ORBIT_TRY(upload(A, &q.phase_off, Q.phase_off));
+    }
   ORBIT_TRY(upload(A, &d.perm, S.perm));
   ORBIT_TRY(upload(A, &d.iperm, S.iperm));
   ORBIT_TRY(upload(A, &d.level, S.level));
@@ -534,6 +541,11 @@ int orbit_factor_create_ex(orbit_symbolic_t sym, int n_orbits, int n_sets, int n
   if ((rc = dalloc(A, &f->Ybuf, (size_t)n_orbits * N))) return fail(rc);
   if ((rc = dalloc(A, &f->Wbuf, (size_t)n_orbits * S.w_size))) return fail(rc);
   if ((rc = dalloc(A, &f->counters, (size_t)n_orbits * 16 * S.nsuper))) return fail(rc);
+  if (S.max_sub_front == 0) {
+    f->flow_bytes = 2 * vb * (size_t)n_orbits * (S.w_size + 2 * N);
+    if ((rc = dalloc(A, &f->flow, f->flow_bytes))) return fail(rc);
+    if (cudaMemset(f->flow, 0, f->flow_bytes) != cudaSuccess) return fail(ORBIT_ERR_CUDA);
+  }
   if ((rc = dalloc(A, &f->E, (size_t)n_orbits * 8 * N))) return fail(rc);
   if ((rc = dalloc(A, &f->tmpv, (size_t)n_orbits * 23 * N))) return fail(rc);
   if ((rc = dalloc(A, &f->orbit_ids, (size_t)n_orbits))) return fail(rc);

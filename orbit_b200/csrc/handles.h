@@ -24,6 +24,10 @@ struct DevSym {
     int32_t *phase_off = nullptr, *phase_offT = nullptr;
     int32_t *nchunk_fwd = nullptr, *nchunk_bwd = nullptr, *nchunk_fwdT = nullptr, *nchunk_bwdT = nullptr;
   } sched[orbit::kNumSched];
+  struct Flow {
+    orbit::FlowRec *recs = nullptr;
+    int32_t *phase_off = nullptr;
+  } staged[orbit::kNumSched][2], columns[orbit::kNumSched];
   int32_t *perm = nullptr, *iperm = nullptr;
   int32_t *level = nullptr;
   int64_t *tc_pack_off = nullptr;
@@ -69,6 +73,11 @@ struct orbit_factor_s {
   double* Ybuf = nullptr;   // N
   double* Wbuf = nullptr;   // w_size
   int* counters = nullptr;  // 8 * 2 * nsuper
+  // tagged results of the dataflow chain kernels, all orbits: w_size update
+  // entries, N forward results and N solutions each
+  unsigned char* flow = nullptr;
+  size_t flow_bytes = 0;
+  unsigned flow_seq = 0;    // launches so far (28 bits), the tags' high part
   double* E = nullptr;      // 8 N forcing (new order)
   double* tmpv = nullptr;   // 4 N scratch vectors
   int* orbit_ids = nullptr; // n_orbits

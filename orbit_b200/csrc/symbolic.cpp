@@ -211,6 +211,14 @@ std::string build_symbolic(int nz, int ny, int nx, const SymbolicOptions& opt, S
   for (int s = 0; s < ns; ++s)
     for (int64_t q = S.uoff[s] + 1; q < S.uoff[s + 1]; ++q)
       if (S.rel[q] <= S.rel[q - 1]) return "internal: extend-add map not increasing";
+  // a child touches every unknown of its parent's separator: the chained
+  // solve reuses its buffers from bin to bin on the strength of this
+  for (int s = 0; s < ns; ++s) {
+    const int p = S.parent[s];
+    if (p < 0) continue;
+    if (S.m[s] < S.n[p] || S.rel[S.uoff[s] + S.n[p] - 1] != S.n[p] - 1)
+      return "internal: a child does not touch its parent's whole separator";
+  }
   S.ginv_off.assign(ns + 1, 0);
   for (int s = 0; s < ns; ++s) S.ginv_off[s + 1] = S.ginv_off[s] + 2 * int64_t(S.n[s] + S.m[s]);
   S.ginv.assign(S.ginv_off[ns], -1);
@@ -624,6 +632,81 @@ std::string build_symbolic(int nz, int ny, int nx, const SymbolicOptions& opt, S
     Q.phase_offT.push_back(int32_t(Q.sitems.size() / 4) - base);
     Q.items_per_binT = Q.phase_offT.back();
   }
+  auto flow_rec = [&](int s, int r0, int r1, int kind, int len) {
+    FlowRec r;
+    r.s = s; r.r0 = r0; r.r1 = r1; r.kind_len = kind + 256 * len;
+    r.n = S.n[s]; r.m = S.m[s]; r.first = S.first[s]; r.ldn = S.ldn[s]; r.ldm = S.ldm[s];
+    r.woff = int32_t(S.woff[s]);
+    const int c0 = S.child[2 * s], c1 = S.child[2 * s + 1];
+    r.w0 = c0 >= 0 ? int32_t(S.woff[c0]) : -1;
+    r.w1 = c1 >= 0 ? int32_t(S.woff[c1]) : -1;
+    r.fac_off = S.fac_off[s];
+    r.map_off = (kind & 1) == 0 ? S.ginv_off[s] : S.uoff[s];
+    return r;
+  };
+  // Column chunks of the transposed dataflow sweeps: vectors of consecutive
+  // columns, so a chunk starts at a multiple of 32 columns of its block (SQ
+  // below column n, Qr from n on; of 16 in the small-batch schedule, whose chunks
+  // at the tree's top would be too few otherwise) and does not straddle the two.
+  for (int k = 0; k < kNumSched && S.max_sub_front == 0; ++k) {
+    FlowSched& P = S.columns[k];
+    const int64_t elems = S.sched[k].chunk_elems;
+    const int grain = k == 0 ? 16 : 32;
+    auto chunks = [&](int s, int kind) {
+      const int n = S.n[s], m = S.m[s], cols = kind == 2 ? n + m : n;
+      int64_t acc = 0;
+      for (int c = 0, start = 0; c < cols; ++c) {
+        acc += (kind == 2 ? std::min(c + 1, n) : n - c + m) + 8;
+        const int at = c + 1 - (c >= n ? n : 0);
+        if ((acc >= elems && at % grain == 0) || c == n - 1 || c == cols - 1) {
+          P.recs.push_back(flow_rec(s, start, c + 1, kind, 0));
+          start = c + 1;
+          acc = 0;
+        }
+      }
+    };
+    for (int l = S.nlevels - 1; l >= 0; --l) {
+      P.phase_off.push_back(int32_t(P.recs.size()));
+      for (int s : S.level_sups[l]) chunks(s, 2);
+    }
+    for (int l = 0; l < S.nlevels; ++l) {
+      P.phase_off.push_back(int32_t(P.recs.size()));
+      for (int s : S.level_sups[l]) chunks(s, 3);
+    }
+    P.phase_off.push_back(int32_t(P.recs.size()));
+    P.items_per_bin = P.phase_off.back();
+  }
+  for (int k = 0; k < kNumSched && S.max_sub_front == 0; ++k)
+    for (int prec = 0; prec < 2; ++prec) {
+      const SolveSched& Q = S.sched[k];
+      FlowSched& P = S.staged[k][prec];
+      const int64_t vb = prec ? 8 : 4;
+      size_t ph = 0;
+      for (int32_t i = 0; i < Q.items_per_bin; ++i) {
+        while (ph < Q.phase_off.size() && Q.phase_off[ph] == i) {
+          P.phase_off.push_back(int32_t(P.recs.size()));
+          ++ph;
+        }
+        const int32_t* it = Q.sitems.data() + 4 * size_t(i);
+        const int s = it[0], kind = it[3], n = S.n[s], m = S.m[s];
+        const int len = kind == 0 ? std::min(it[2] - 1, n) : n - it[1] + m;
+        for (int a = it[1]; a < it[2];) {
+          int b = a + 1;
+          while (b < it[2]) {
+            const int64_t full = (b + 1 - a) * staged_row(kind, a, b + 1, n, S.ldn[s], S.ldm[s]) * vb;
+            if (full > kStageBytes || (full > kStageBytesCut && b - a >= 4)) break;
+            ++b;
+          }
+          P.recs.push_back(flow_rec(s, a, b, kind, len));
+          a = b;
+        }
+      }
+      while (ph < Q.phase_off.size()) {
+        P.phase_off.push_back(int32_t(P.recs.size()));
+        ++ph;
+      }
+      P.items_per_bin = P.phase_off.back();
+    }
   return std::string();
 }
 

@@ -40,6 +40,18 @@ inline int64_t front_smem_elems(int64_t n, int64_t m) {
 
 inline int64_t round_up(int64_t a, int64_t b) { return (a + b - 1) / b * b; }
 
+// Elements between the staged rows of a row chunk [a, b) (kind 0 forward: row i
+// of [SQ; Pb] up to column min(i, n); kind 1 backward: the SQ row from column a
+// on, rounded down to 4, then the Qr row).
+inline
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+int64_t staged_row(int kind, int a, int b, int n, int ldn, int ldm) {
+  const int last = b - 1 < n ? b - 1 : n;
+  return kind == 0 ? (last + 3) / 4 * 4 : int64_t(ldn - a / 4 * 4) + ldm;
+}
+
 // One kernel launch of the numeric factorization schedule.
 struct FactorLaunch {
   enum Kind : int { ZERO = 0, SCATTER, EXTEND, DIAG, PANEL, UPDATE, SCHUR, INV, TRIL, PRODL, TRIU, PRODU, TC_PACK, ASSEMBLE, TC_GEMM, FRONT } kind;
@@ -63,6 +75,27 @@ struct SolveSched {
   std::vector<int32_t> nchunk_fwd, nchunk_bwd, nchunk_fwdT, nchunk_bwdT;
 };
 constexpr int kNumSched = 3;
+// Shared-memory staging of the chained solve: bytes of factor rows that one
+// staged task holds at most, and the size it is cut to where that leaves a row
+// for each of its block's warps.
+constexpr int kStageBytes = 24576;
+constexpr int kStageBytesCut = 12288;
+
+// One task of the dataflow kernel, with what its supernode's arrays say.
+struct FlowRec {
+  int32_t s, r0, r1;
+  int32_t kind_len;  // kind + 256 * len; len: row length that the lanes per row follow from (kinds 0, 1)
+  int32_t n, m, first, ldn, ldm, woff;
+  int32_t w0, w1;    // update offsets of the children (-1: none)
+  int64_t fac_off;
+  int64_t map_off;   // forward kinds (0, 2): ginv offset; backward (1, 3): uidx offset
+};
+static_assert(sizeof(FlowRec) == 64, "loaded as four 16-byte vectors");
+struct FlowSched {
+  std::vector<FlowRec> recs;
+  std::vector<int32_t> phase_off;
+  int32_t items_per_bin = 0;
+};
 
 struct Symbolic {
   int nz = 0, ny = 0, nx = 0;
@@ -104,6 +137,12 @@ struct Symbolic {
   std::vector<int32_t> fitems;            // 4 ints per item
   std::vector<FactorLaunch> fsched;
   SolveSched sched[kNumSched];  // chunk/2, chunk, 2 chunk; sched[1] is the default
+  // the non-transposed chunks of sched[k] cut into staged tasks, for FP32 (0)
+  // and FP64 (1) factors.  A row keeps the lanes of its uncut chunk, and with
+  // them the order of its sum.
+  FlowSched staged[kNumSched][2];
+  // their transposed counterparts (column chunks, both precisions)
+  FlowSched columns[kNumSched];
   std::vector<int32_t> role;  // 0 chunked node, 1 subtree-task root, 2 inside a subtree
   int max_front = 0;
   int max_sub_front = 0;  // largest n+m of a supernode inside a subtree task
