@@ -137,12 +137,18 @@ int build_device_symbolic(orbit_symbolic_s* h) {
     ORBIT_TRY(upload(A, &q.nchunk_bwdT, Q.nchunk_bwdT));
   }
   for (int k = 0; k < kNumSched && S.max_sub_front == 0; ++k)
-    for (int v = 0; v < 3; ++v) {
-      const FlowSched& Q = v < 2 ? S.staged[k][v] : S.columns[k];
-      DevSym::Flow& q = v < 2 ? d.staged[k][v] : d.columns[k];
+    for (int v = 0; v < 4; ++v) {
+      const FlowSched& Q = v < 2 ? S.staged[k][v] : v == 2 ? S.columns[k] : S.whole[k];
+      DevSym::Flow& q = v < 2 ? d.staged[k][v] : v == 2 ? d.columns[k] : d.whole[k];
       ORBIT_TRY(upload(A, &q.recs, Q.recs));
       ORBIT_TRY(upload(A, &q.phase_off, Q.phase_off));
     }
+  if (S.max_sub_front == 0) {
+    ORBIT_TRY(upload(A, &d.wide.recs, S.wide.recs));
+    ORBIT_TRY(upload(A, &d.wide.phase_off, S.wide.phase_off));
+    ORBIT_TRY(upload(A, &d.wide_nch_f, S.wide_nch_f));
+    ORBIT_TRY(upload(A, &d.wide_nch_b, S.wide_nch_b));
+  }
   ORBIT_TRY(upload(A, &d.perm, S.perm));
   ORBIT_TRY(upload(A, &d.iperm, S.iperm));
   ORBIT_TRY(upload(A, &d.level, S.level));
@@ -545,6 +551,10 @@ int orbit_factor_create_ex(orbit_symbolic_t sym, int n_orbits, int n_sets, int n
     f->flow_bytes = 2 * vb * (size_t)n_orbits * (S.w_size + 2 * N);
     if ((rc = dalloc(A, &f->flow, f->flow_bytes))) return fail(rc);
     if (cudaMemset(f->flow, 0, f->flow_bytes) != cudaSuccess) return fail(ORBIT_ERR_CUDA);
+    if (precision == ORBIT_PREC_FP32 && n_sets == 1 && n_orbits > 1) {
+      // whole groups of 16, 8 or 4: fewer than twice the orbits
+      if ((rc = dalloc(A, &f->multi, (size_t)2 * n_orbits * (S.w_size + 2 * N)))) return fail(rc);
+    }
   }
   if ((rc = dalloc(A, &f->E, (size_t)n_orbits * 8 * N))) return fail(rc);
   if ((rc = dalloc(A, &f->tmpv, (size_t)n_orbits * 23 * N))) return fail(rc);

@@ -27,7 +27,8 @@ struct DevSym {
   struct Flow {
     orbit::FlowRec *recs = nullptr;
     int32_t *phase_off = nullptr;
-  } staged[orbit::kNumSched][2], columns[orbit::kNumSched];
+  } staged[orbit::kNumSched][2], columns[orbit::kNumSched], whole[orbit::kNumSched], wide;
+  int32_t *wide_nch_f = nullptr, *wide_nch_b = nullptr;
   int32_t *perm = nullptr, *iperm = nullptr;
   int32_t *level = nullptr;
   int64_t *tc_pack_off = nullptr;
@@ -77,6 +78,8 @@ struct orbit_factor_s {
   // entries, N forward results and N solutions each
   unsigned char* flow = nullptr;
   size_t flow_bytes = 0;
+  // interleaved results of the FP32 many-right-hand-side kernels
+  float* multi = nullptr;
   unsigned flow_seq = 0;    // launches so far (28 bits), the tags' high part
   double* E = nullptr;      // 8 N forcing (new order)
   double* tmpv = nullptr;   // 4 N scratch vectors

@@ -1197,13 +1197,13 @@ __device__ __forceinline__ void stage16(void* dst, const void* src, uint64_t pol
 // Stages columns [c0(r), c1(r)) of the rows r = 0 .. rows - 1 of a row-major
 // block (16-byte aligned bounds, in vectors; at most nv of them), row r at
 // dst + r * stride; as many lanes per row as it has vectors, up to a warp.
-template <typename T, typename C0, typename C1>
+template <typename T, int NW, typename C0, typename C1>
 __device__ __forceinline__ void stage_rows(T* dst, int stride, const T* src, int64_t ld, int rows, int nv,
                                            uint64_t pol, C0&& c0, C1&& c1) {
   constexpr int W = Vec16<T>::w;
   const int lg = nv >= 32 ? 5 : nv <= 1 ? 0 : 32 - __clz(nv - 1);
   const int per = 32 >> lg, lane = threadIdx.x & 31, gl = lane & ((1 << lg) - 1);
-  for (int r = (threadIdx.x >> 5) * per + (lane >> lg); r < rows; r += kWarps * per) {
+  for (int r = (threadIdx.x >> 5) * per + (lane >> lg); r < rows; r += NW * per) {
     const T* a = src + (int64_t)r * ld;
     T* d = dst + r * stride;
     for (int k = c0(r) + gl; k < c1(r); k += 1 << lg) stage16(d + k * W, a + k * W, pol);
@@ -1212,38 +1212,37 @@ __device__ __forceinline__ void stage_rows(T* dst, int stride, const T* src, int
 
 // A block's claimed task: index (the launch's total or more: none), bin in
 // claim order, orbit, its factor set, and the task's record.
-struct FlowClaim {
+struct __align__(16) FlowClaim {  // written as 16-byte vectors
   FlowRec rec;
-  int t, q, o, set;
+  int t, q, gi, o, set;
 };
 
-// Warp 0 claims the next task and writes it to shared memory; ends with a
-// block barrier.  slot: of the last claimed task.
+// A whole warp claims the next task and writes it to shared memory.  slot: of
+// the last claimed task; K right-hand sides per group.
 template <typename T>
-__device__ __forceinline__ void flow_claim(const ChainDev<T>& D, const SlotTables& tab, FlowClaim& c, int& slot) {
-  const int tid = threadIdx.x;
-  if (tid < 32) {
-    int t = 0;
-    if (tid == 0) {
-      t = atomicAdd(D.task_counter, 1);
-      if (ld_volatile(D.status) != 0) t = D.total;
-    }
-    t = __shfl_sync(0xffffffffu, t, 0);
-    if (t < D.total) {
-      while (tab.slot[slot + 1] <= t) ++slot;
-      int q, ph, gi, item;
-      slot_task(D, tab, t, slot, q, ph, gi, item);
-      if (tid < 4) reinterpret_cast<int4*>(&c.rec)[tid] = __ldg(reinterpret_cast<const int4*>(D.recs + item) + tid);
-      if (tid == 4) {
-        const int o = D.orbit_ids[gi];
-        c.q = q;
-        c.o = o;
-        c.set = D.set_of[o];
-      }
-    }
-    if (tid == 5) c.t = t;
+__device__ __forceinline__ void flow_claim(const ChainDev<T>& D, const SlotTables& tab, FlowClaim& c, int& slot,
+                                           int K = 1) {
+  const int lane = threadIdx.x & 31;
+  int t = 0;
+  if (lane == 0) {
+    t = atomicAdd(D.task_counter, 1);
+    if (ld_volatile(D.status) != 0) t = D.total;
   }
-  __syncthreads();
+  t = __shfl_sync(0xffffffffu, t, 0);
+  if (t < D.total) {
+    while (tab.slot[slot + 1] <= t) ++slot;
+    int q, ph, gi, item;
+    slot_task(D, tab, t, slot, q, ph, gi, item);
+    if (lane < 4) reinterpret_cast<int4*>(&c.rec)[lane] = __ldg(reinterpret_cast<const int4*>(D.recs + item) + lane);
+    if (lane == 4) {
+      const int o = D.orbit_ids[gi * K];
+      c.q = q;
+      c.gi = gi;
+      c.o = o;
+      c.set = D.set_of[o];
+    }
+  }
+  if (lane == 5) c.t = t;
 }
 
 // Row-oriented sweeps of launches bound by their dependency chain.  A task's
@@ -1269,7 +1268,8 @@ __global__ void __launch_bounds__(kSolveThreads, 5)
   build_slots(D, s_tab);
   const uint64_t pol = stream_policy(D.stream_ef != 0);
   for (int slot = 0;;) {
-    flow_claim(D, s_tab, s_claim, slot);
+    if (tid < 32) flow_claim(D, s_tab, s_claim, slot);
+    __syncthreads();
     const int t = s_claim.t;
     if (t >= D.total) break;
     const int tau = D.tau0 + s_claim.q, o = s_claim.o;
@@ -1283,13 +1283,13 @@ __global__ void __launch_bounds__(kSolveThreads, 5)
     const int a0 = r0 & ~3;  // first staged column of a backward task
     if (staged) {
       if (kind == 0) {
-        stage_rows(stage, stride, SQ + (int64_t)r0 * ldn, ldn, r1 - r0, stride / W, pol, [](int) { return 0; },
+        stage_rows<T, kWarps>(stage, stride, SQ + (int64_t)r0 * ldn, ldn, r1 - r0, stride / W, pol, [](int) { return 0; },
                    [&](int r) { return (min(r0 + r, n) + W - 1) / W; });
       } else {
-        stage_rows(stage, stride, SQ + (int64_t)r0 * ldn + a0, ldn, r1 - r0, (ldn - a0) / W, pol,
+        stage_rows<T, kWarps>(stage, stride, SQ + (int64_t)r0 * ldn + a0, ldn, r1 - r0, (ldn - a0) / W, pol,
                    [&](int r) { return (r0 + r - a0) / W; }, [&](int) { return (n - a0 + W - 1) / W; });
         if (m > 0)
-          stage_rows(stage + ldn - a0, stride, Qr + (int64_t)r0 * ldm, ldm, r1 - r0, ldm / W, pol,
+          stage_rows<T, kWarps>(stage + ldn - a0, stride, Qr + (int64_t)r0 * ldm, ldm, r1 - r0, ldm / W, pol,
                      [](int) { return 0; }, [&](int) { return (m + W - 1) / W; });
       }
     }
@@ -1370,7 +1370,8 @@ __global__ void __launch_bounds__(kSolveThreads, 7) k_flow_t(ChainDev<T> D) {
   build_slots(D, s_tab);
   const uint64_t pol = stream_policy(D.stream_ef != 0);
   for (int slot = 0;;) {
-    flow_claim(D, s_tab, s_claim, slot);
+    if (tid < 32) flow_claim(D, s_tab, s_claim, slot);
+    __syncthreads();
     const int t = s_claim.t;
     if (t >= D.total) break;
     const int tau = D.tau1 - 1 - s_claim.q, o = s_claim.o;
@@ -1713,6 +1714,646 @@ __global__ void __launch_bounds__(kSolveThreads, sizeof(T) == 4 ? ORBIT_SOLVE_MI
   }
 }
 
+// ---- many right-hand sides on one FP32 factor set ----
+//
+// K right-hand sides (4, 8 or 16) per task, interleaved: update entries,
+// forward results and solutions are handed on as [position][K] floats, so that
+// a gather reads one position's K values with 16-byte loads, and a factor value
+// read once is used K times.  Bound by the shared-memory reads of the K vectors
+// (16 bytes per 4 multiply-adds and row): four rows (or two columns) per lane
+// share each of them, and the multiply-adds run two right-hand sides per
+// instruction.  Every right-hand side's sums have the order of the kernels
+// with four of them per task (k_chain_multi), whatever K is.
+//
+// What is left is per-task latency (claim, wait, gather: 6 of a task's 12 us) at
+// two blocks per SM, which the vectors of the largest fronts allow.  80x72x15
+// grid, 8 bins, 64 right-hand sides, a sweep against groups of four with one row
+// (column) per lane: 18.0 -> 8.0 ms, transposed 17.4 -> 9.0 ms.
+constexpr int kMultiThreads = 256;
+constexpr int kMultiWarps = kMultiThreads / 32;
+constexpr size_t kMultiSmem = 108 * 1024;  // two blocks per SM
+
+struct MultiDev {
+  ChainDev<float> C;
+  float *W, *Y, *X;  // per group w_size x K, N x K, N x K
+  const int32_t *nch_f, *nch_b;
+  int smem_floats;  // dynamic shared memory of a block
+};
+
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+  unsigned long long d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+  return d;
+}
+__device__ __forceinline__ void unpack2(unsigned long long d, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(d));
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
+// 16-byte chunk (right-hand sides 4 kq .. 4 kq + 3) of position j in the shared
+// vectors: blocks of four positions, the chunks of a block permuted so that
+// lanes reading the same chunk of eight consecutive blocks meet no bank twice.
+template <int K>
+__device__ __forceinline__ int multi_chunk(int j, int kq) {
+  constexpr int QC = K / 4;
+  const int jq = j >> 2, c = (j & 3) * QC + kq;
+  return jq * 4 * QC + (QC == 1 ? c ^ ((jq >> 1) & 3) : c ^ (jq & 7));
+}
+
+// Forward right-hand side of the positions [0, min(r1, n)) and, from position
+// `low` on, [max(r0, n), r1): own entries of the previous bin's solution (or of
+// the launch's input) plus forcing and the children's update entries, K vectors.
+template <int K, bool TR>
+__device__ __forceinline__ void multi_gather_fwd(const MultiDev& M, const FlowRec& R, int gi, const int* o, int tau,
+                                                 int r0, int r1, int low, float4* V) {
+  const ChainDev<float>& D = M.C;
+  constexpr int QC = K / 4;
+  const int n = R.n, first = R.first, w = n + R.m;
+  const bool first_bin = TR ? tau == D.tau1 - 1 : tau == D.tau0;
+  const int bin_in = TR ? tau + 1 : tau;
+  const int bin_e = TR ? tau + 1 : tau;
+  const bool forced = D.E && (!TR || tau + 1 < D.tau1);
+  const float4* Xg = reinterpret_cast<const float4*>(M.X + (int64_t)gi * D.N * K) + (int64_t)first * QC;
+  const float4* Wg = reinterpret_cast<const float4*>(M.W + (int64_t)gi * D.w_size * K);
+  const int32_t* g0 = D.ginv + R.map_off;
+  const float4* W0 = Wg + (int64_t)max(R.w0, 0) * QC;
+  const float4* W1 = Wg + (int64_t)max(R.w1, 0) * QC;
+  const int lo_end = min(r1, n), hi0 = max(r0, n);
+  const int cnt = lo_end + max(0, r1 - hi0);
+#pragma unroll 2
+  for (int idx = threadIdx.x; idx < cnt * QC; idx += kMultiThreads) {
+    const int q = idx / QC, kq = idx % QC;
+    const int i = q < lo_end ? q : q - lo_end + hi0;
+    const int u0 = g0[i], u1 = g0[w + i];
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f), a = x, b = x;
+    if (u0 >= 0) a = __ldcg(W0 + (int64_t)u0 * QC + kq);
+    if (u1 >= 0) b = __ldcg(W1 + (int64_t)u1 * QC + kq);
+    if (i < n) {
+      if (first_bin) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = D.X[((int64_t)o[4 * kq + k] * 9 + bin_in) * D.N + first + i];
+      } else {
+        x = __ldcg(Xg + (int64_t)i * QC + kq);
+        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+      }
+      if (forced)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] += D.escale * D.E[((int64_t)o[4 * kq + k] * 8 + bin_e) * D.N + first + i];
+    }
+    if (u0 >= 0) { v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w; }
+    if (u1 >= 0) { v[0] += b.x; v[1] += b.y; v[2] += b.z; v[3] += b.w; }
+    V[multi_chunk<K>(q < lo_end ? q : low + q - lo_end, kq)] = make_float4((float)v[0], (float)v[1], (float)v[2], (float)v[3]);
+  }
+}
+
+// Positions [at, at + cnt) of the shared vectors from [position][K] arrays:
+// src + idx(q) for q < cnt.
+template <int K, typename Idx>
+__device__ __forceinline__ void multi_gather(const float* src, int at, int cnt, float4* V, Idx&& idx) {
+  constexpr int QC = K / 4;
+  const float4* s4 = reinterpret_cast<const float4*>(src);
+#pragma unroll 4
+  for (int e = threadIdx.x; e < cnt * QC; e += kMultiThreads) {
+    const int q = e / QC, kq = e % QC;
+    V[multi_chunk<K>(at + q, kq)] = __ldcg(s4 + (int64_t)idx(q) * QC + kq);
+  }
+}
+
+// acc[r][:] += (4 factor values a[r] of one vector) . (block jq of the shared
+// vectors) for NR rows and the KW right-hand sides from 4 k0 on.  The value pairs
+// of the factor entries are formed once for all of them.
+template <int K, int KW, int NR>
+__device__ __forceinline__ void multi_block(const float4* V, int jq, int k0, const float4 (&a)[NR],
+                                            unsigned long long (&acc)[NR][KW / 2]) {
+  unsigned long long p[NR][4];
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    p[r][0] = pack2(a[r].x, a[r].x);
+    p[r][1] = pack2(a[r].y, a[r].y);
+    p[r][2] = pack2(a[r].z, a[r].z);
+    p[r][3] = pack2(a[r].w, a[r].w);
+  }
+#pragma unroll
+  for (int kq = 0; kq < KW / 4; ++kq) {
+    unsigned long long v[4][2];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(V + multi_chunk<K>(4 * jq + j, k0 + kq));
+      v[j][0] = t.x;
+      v[j][1] = t.y;
+    }
+#pragma unroll
+    for (int r = 0; r < NR; ++r)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        acc[r][2 * kq + h] =
+            add2(acc[r][2 * kq + h],
+                 fma2(p[r][3], v[3][h], fma2(p[r][2], v[2][h], fma2(p[r][0], v[0][h], mul2(p[r][1], v[1][h])))));
+  }
+}
+
+// acc[:] += x v[j] for one position j.
+template <int K, int KW>
+__device__ __forceinline__ void multi_one(const float4* V, int j, int k0, float x, unsigned long long (&acc)[KW / 2]) {
+  const unsigned long long xx = pack2(x, x);
+#pragma unroll
+  for (int kq = 0; kq < KW / 4; ++kq) {
+    const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(V + multi_chunk<K>(j, k0 + kq));
+    acc[2 * kq] = fma2(xx, t.x, acc[2 * kq]);
+    acc[2 * kq + 1] = fma2(xx, t.y, acc[2 * kq + 1]);
+  }
+}
+
+// Sums over the G lanes of a group, the pairs of a butterfly, each lane keeping
+// its share: values [4 rows][K] flat, on return 4 K / G of them from index
+// `base` on.
+template <int G, int K>
+__device__ __forceinline__ int multi_reduce(unsigned long long (&acc)[4][K / 2], int gl, float (&v)[4 * K]) {
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int h = 0; h < K / 2; ++h) unpack2(acc[r][h], v[r * K + 2 * h], v[r * K + 2 * h + 1]);
+  int base = 0;
+  int cnt = 4 * K;
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1) {
+    // below one value per lane the rest of the group adds up the same values
+    if (cnt > 1) {
+      cnt >>= 1;
+      const bool up = (gl & o) != 0;
+#pragma unroll
+      for (int q = 0; q < 2 * K; ++q)
+        if (q < cnt) {
+          const float mine = up ? v[q + cnt] : v[q], other = up ? v[q] : v[q + cnt];
+          v[q] = mine + __shfl_xor_sync(0xffffffffu, other, o);
+        }
+      base += up ? cnt : 0;
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    }
+  }
+  return base;
+}
+
+// Row quads [4 q, 4 q + 4) of a task's rows [b0, b1), G lanes each; column j of
+// row i at A0[(i - b0) * lda + j], of its ancestors' panel at B0[(i - b0) * ldb + j]
+// (staged, or in global memory).  Forward: vectors from position 0, the rows'
+// own values beyond n at `low`, from row `own0` on.  Backward: vectors of the
+// own part at position j - at0, of the ancestors at `low`.
+template <int G, int K, bool FWD>
+__device__ __forceinline__ void multi_rows(const MultiDev& M, const FlowRec& R, int gi, const int* o, int nk, int tau,
+                                           int b0, int b1, const float* A0, int lda, const float* B0, int ldb, int at0,
+                                           int low, int own0, const float4* V) {
+  const ChainDev<float>& D = M.C;
+  const int n = R.n, m = R.m, first = R.first;
+  // a warp takes up to 8 of the right-hand sides
+  constexpr int KW = K < 8 ? K : 8, HALVES = K / KW;
+  const int lane = threadIdx.x & 31, gl = lane & (G - 1), warp = threadIdx.x >> 5;
+  const int k0 = (warp % HALVES) * (KW / 4);
+  constexpr int per = 32 / G, sets = kMultiWarps / HALVES, NV = 4 * KW / G > 0 ? 4 * KW / G : 1;
+  const int q0 = b0 >> 2, q1 = (b1 + 3) >> 2;
+  for (int qb = q0 + (warp / HALVES) * per; qb < q1; qb += sets * per) {
+    const int qd = qb + lane / G, i0 = 4 * qd;
+    unsigned rows = 0;  // of the quad, in this batch; the others' sums are not stored
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      if (i0 + r >= b0 && i0 + r < b1) rows |= 1u << r;
+    unsigned long long acc[4][KW / 2];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int h = 0; h < KW / 2; ++h) acc[r][h] = 0ull;
+    auto quad = [&](const float* p, int ld, int kk, float4 (&a)[4]) {
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        a[r] = (rows >> r) & 1u ? *(reinterpret_cast<const float4*>(p + r * ld) + kk) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    const float* A = A0 + (int64_t)(i0 - b0) * lda;
+    if (FWD) {
+      if (rows) {
+        const int nv1 = min(i0, n) >> 2;  // the quad's rows share their whole vectors
+        for (int kk = gl; kk < nv1; kk += G) {
+          float4 a[4];
+          quad(A, lda, kk, a);
+          multi_block<K, KW, 4>(V, kk, k0, a, acc);
+        }
+        const int j = 4 * nv1 + gl;
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+          if (((rows >> r) & 1u) && j < min(i0 + r, n)) multi_one<K, KW>(V, j, k0, A[r * lda + j], acc[r]);
+      }
+    } else {
+      // Upper triangle: row r's whole vectors start at ceil(i / 4), the quad's
+      // first row one block before the others; lanes are aligned to the
+      // others, and the first row's sums move one lane on afterwards.
+      const int nvn = n >> 2;
+      if (rows) {
+#pragma unroll
+        for (int r = 1; r < 4; ++r) {
+          const int j = i0 + r + gl;
+          if (((rows >> r) & 1u) && j < min(i0 + 4, n)) multi_one<K, KW>(V, j - at0, k0, A[r * lda + j], acc[r]);
+        }
+        if (gl == G - 1 && (rows & 1u) && qd < nvn) {
+          const float4 a1[1] = {*(reinterpret_cast<const float4*>(A) + qd)};
+          unsigned long long c1[1][KW / 2];
+#pragma unroll
+          for (int h = 0; h < KW / 2; ++h) c1[0][h] = acc[0][h];
+          multi_block<K, KW, 1>(V, qd - (at0 >> 2), k0, a1, c1);
+#pragma unroll
+          for (int h = 0; h < KW / 2; ++h) acc[0][h] = c1[0][h];
+        }
+        for (int kk = qd + 1 + gl; kk < nvn; kk += G) {
+          float4 a[4];
+          quad(A, lda, kk, a);
+          multi_block<K, KW, 4>(V, kk - (at0 >> 2), k0, a, acc);
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          // lane of the row's own order that this lane stands for
+          const int jb = max(r == 0 ? i0 : min(i0 + 4, n), nvn * 4), j = jb + (r == 0 ? (gl + 1) & (G - 1) : gl);
+          if (((rows >> r) & 1u) && j < n) multi_one<K, KW>(V, j - at0, k0, A[r * lda + j], acc[r]);
+        }
+      }
+      __syncwarp();
+#pragma unroll
+      for (int h = 0; h < KW / 2; ++h)
+        acc[0][h] = __shfl_sync(0xffffffffu, acc[0][h], (lane & ~(G - 1)) | ((gl - 1) & (G - 1)));
+      if (rows) {
+        const float* B = B0 + (int64_t)(i0 - b0) * ldb;
+        const int nv = m >> 2;
+        for (int kk = gl; kk < nv; kk += G) {
+          float4 a[4];
+          quad(B, ldb, kk, a);
+          multi_block<K, KW, 4>(V, (low >> 2) + kk, k0, a, acc);
+        }
+        const int j = 4 * nv + gl;
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+          if (((rows >> r) & 1u) && j < m) multi_one<K, KW>(V, low + j, k0, B[r * ldb + j], acc[r]);
+      }
+    }
+    __syncwarp();
+    float v[4 * KW];
+    const int base = multi_reduce<G, KW>(acc, gl, v);
+    // this lane's share: NV consecutive right-hand sides of one row
+    const int r = base / KW, k = 4 * k0 + base % KW, i = i0 + r;
+    if ((rows >> r) & 1u) {
+      float* out;
+      if (FWD) {
+        const int at = i < n ? i : low + i - own0;
+#pragma unroll
+        for (int e = 0; e < NV; ++e)
+          v[e] = reinterpret_cast<const float*>(V + multi_chunk<K>(at, (k + e) >> 2))[(k + e) & 3] + v[e];
+        out = i < n ? M.Y + ((int64_t)gi * D.N + first + i) * K + k
+                    : M.W + ((int64_t)gi * D.w_size + R.woff + (i - n)) * K + k;
+      } else {
+        out = M.X + ((int64_t)gi * D.N + first + i) * K + k;
+        double* X = D.X + (int64_t)(tau + 1) * D.N + first + i;
+#pragma unroll
+        for (int e = 0; e < NV; ++e)
+          if (k + e < nk) X[(int64_t)o[k + e] * 9 * D.N] = (double)v[e];
+      }
+      if constexpr (NV >= 4) {
+#pragma unroll
+        for (int e = 0; e < NV; e += 4)
+          *reinterpret_cast<float4*>(out + e) = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+      } else if constexpr (NV == 2) {
+        *reinterpret_cast<float2*>(out) = make_float2(v[0], v[1]);
+      } else {
+        out[0] = v[0];
+      }
+    }
+  }
+}
+
+// Column chains of a transposed task (see flow_chains) for K right-hand sides,
+// VEC columns per lane: rows i0, i0 + 4, ... below i1 of a (at this lane's first
+// column), positions i - at0 of the shared vectors.  DIAG: row i counts for
+// column c + q when i <= c + q (1) or i > c + q (2).
+template <int K, int VEC, int DIAG, int U>
+__device__ __forceinline__ void multi_chain(const float* __restrict__ a, int64_t ld, int c, int i0, int i1,
+                                            const float4* V, int at0, unsigned long long (&acc)[VEC][K / 2]) {
+  using T = typename std::conditional<VEC == 2, float2, float>::type;
+  for (int i = i0; i < i1; i += 4 * U) {
+    T x[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      x[u] = T{};
+      if (u == 0 || i + 4 * u < i1) x[u] = __ldg(reinterpret_cast<const T*>(a + (int64_t)(i + 4 * u) * ld));
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int r = i + 4 * u;
+      if (u == 0 || r < i1) {
+        const float* xe = reinterpret_cast<const float*>(&x[u]);
+#pragma unroll
+        for (int kq = 0; kq < K / 4; ++kq) {
+          const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(V + multi_chunk<K>(r - at0, kq));
+#pragma unroll
+          for (int q = 0; q < VEC; ++q) {
+            const unsigned long long xx = pack2(xe[q], xe[q]);
+            const unsigned long long s0 = fma2(xx, t.x, acc[q][2 * kq]), s1 = fma2(xx, t.y, acc[q][2 * kq + 1]);
+            const bool in = DIAG == 0 || (DIAG == 1 ? r <= c + q : r > c + q);
+            if (in) {
+              acc[q][2 * kq] = s0;
+              acc[q][2 * kq + 1] = s1;
+            }
+          }
+        }
+      }
+    }
+  }
+}
+
+// Transposed task: columns [r0, r1) in pairs of blocks of 32 VEC, the first of a
+// pair by warps 0-3, the second by warps 4-7, warp w of a half on the rows
+// congruent to w.  The chains change warps, and are added up, through the
+// shared memory behind the vectors, or over them where that is full (then the
+// task is one pair, and a backward one gathers the ancestors' solution once its
+// own part is used up).
+template <int K, int VEC>
+__device__ __forceinline__ void multi_cols(const MultiDev& M, const FlowRec& R, int gi, const int* o, int nk, int tau,
+                                           const float* SQ, float4* V) {
+  const ChainDev<float>& D = M.C;
+  constexpr int CB = 32 * VEC, U = 8, QC = K / 4;  // U 4 / 8 / 12 / 16 / 32: 9.3 / 8.2 / 8.4 / 8.7 / 12.5 ms a sweep
+  const bool fwd = R.kind_len == 2;
+  const int r0 = R.r0, r1 = R.r1, n = R.n, m = R.m, first = R.first, ldn = R.ldn, ldm = R.ldm;
+  const int lane = threadIdx.x & 31, half = threadIdx.x >> 7, w = (threadIdx.x >> 5) & 3, ht = threadIdx.x & 127;
+  const int at0 = fwd ? 0 : r0 & ~3;
+  const int low = fwd ? 0 : (n - at0 + 3) & ~3;  // ancestors' part, where it has room of its own
+  const int blocks = (((fwd ? min(r1, n) : low + m) + 3) >> 2) * K;  // 16-byte chunks of all vectors
+  const bool both = (blocks + 2 * 4 * QC * CB) * 4 <= M.smem_floats;
+  // [class][right-hand-side quad][column] of this half
+  ulonglong2* red = reinterpret_cast<ulonglong2*>(both ? V + blocks : V) + half * 4 * QC * CB;
+  const float* Yg = M.Y + ((int64_t)gi * D.N + first) * K;
+  const float* Xg = M.X + (int64_t)gi * D.N * K;
+  const int32_t* ui = D.uidx + (fwd ? 0 : R.map_off);
+  if (fwd) multi_gather_fwd<K, true>(M, R, gi, o, tau, 0, min(r1, n), 0, V);
+  else multi_gather<K>(Yg, r0 - at0, n - r0, V, [&](int q) { return r0 + q; });
+  if (!fwd && both) multi_gather<K>(Xg, low, m, V, [&](int q) { return ui[q]; });
+  __syncthreads();
+  auto from = [&](int i) { return i + ((w - i) & 3); };
+  for (int pair = r0; pair < r1; pair += 2 * CB) {
+  const int cb = pair + half * CB;
+  const bool on = cb < r1;
+  const int cend = min(cb + CB, r1), c = cb + lane * VEC;
+  unsigned long long acc[VEC][K / 2];
+#pragma unroll
+  for (int q = 0; q < VEC; ++q)
+#pragma unroll
+    for (int h = 0; h < K / 2; ++h) acc[q][h] = 0ull;
+  if (fwd) {
+    if (on && c < cend) {
+      if (cb < n) {
+        multi_chain<K, VEC, 0, U>(SQ + c, ldn, c, w, cb, V, 0, acc);
+        multi_chain<K, VEC, 1, U>(SQ + c, ldn, c, from(cb), cend, V, 0, acc);
+      } else {
+        multi_chain<K, VEC, 0, U>(SQ + (int64_t)(n + m) * ldn + (c - n), ldm, c, w, n, V, 0, acc);
+      }
+    }
+  } else {
+    const int d1 = min(cb + CB, n);
+    if (on && c < cend) {
+      multi_chain<K, VEC, 2, U>(SQ + c, ldn, c, from(cb + 1), d1, V, at0, acc);
+      multi_chain<K, VEC, 0, U>(SQ + c, ldn, c, from(d1), n, V, at0, acc);
+    }
+    if (!both) __syncthreads();
+    // the triangle's chain (w - c - 1) mod 4 of a column goes on in that warp
+#pragma unroll
+    for (int kq = 0; kq < QC; ++kq)
+#pragma unroll
+      for (int q = 0; q < VEC; ++q)
+        red[(((w - c - q - 1) & 3) * QC + kq) * CB + lane * VEC + q] = make_ulonglong2(acc[q][2 * kq], acc[q][2 * kq + 1]);
+    __syncthreads();
+#pragma unroll
+    for (int kq = 0; kq < QC; ++kq)
+#pragma unroll
+      for (int q = 0; q < VEC; ++q) {
+        const ulonglong2 t = red[(w * QC + kq) * CB + lane * VEC + q];
+        acc[q][2 * kq] = t.x;
+        acc[q][2 * kq + 1] = t.y;
+      }
+    if (!both) {
+      __syncthreads();
+      multi_gather<K>(Xg, 0, m, V, [&](int q) { return ui[q]; });
+      __syncthreads();
+    }
+    // position of ancestor row i is i (+ low)
+    if (on && c < cend)
+      multi_chain<K, VEC, 0, U>(SQ + (int64_t)n * ldn + c, ldn, c, w, m, V, both ? -low : 0, acc);
+  }
+  if (!both) __syncthreads();
+  // the four chains of a column, added in order to its own value
+#pragma unroll
+  for (int kq = 0; kq < QC; ++kq)
+#pragma unroll
+    for (int q = 0; q < VEC; ++q)
+      red[(w * QC + kq) * CB + lane * VEC + q] = make_ulonglong2(acc[q][2 * kq], acc[q][2 * kq + 1]);
+  __syncthreads();
+  const float4* part = reinterpret_cast<const float4*>(red);
+  const int32_t* g0 = D.ginv + (fwd ? R.map_off : 0);
+  for (int e = on ? ht : CB * QC; e < CB * QC; e += 128) {
+    const int cc = cb + e / QC, kq = e % QC;
+    if (cc >= cend) continue;
+    float4* Y = reinterpret_cast<float4*>(M.Y + ((int64_t)gi * D.N + first + cc) * K) + kq;
+    float4 sum = fwd ? make_float4(0.f, 0.f, 0.f, 0.f) : __ldcg(Y);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float4 t = part[(q * QC + kq) * CB + cc - cb];
+      sum.x += t.x; sum.y += t.y; sum.z += t.z; sum.w += t.w;
+    }
+    if (!fwd) {
+      *(reinterpret_cast<float4*>(M.X + ((int64_t)gi * D.N + first + cc) * K) + kq) = sum;
+      double* X = D.X + (int64_t)tau * D.N + first + cc;
+      const float x[4] = {sum.x, sum.y, sum.z, sum.w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (4 * kq + k < nk) X[(int64_t)o[4 * kq + k] * 9 * D.N] = (double)x[k];
+    } else if (cc < n) {
+      *Y = sum;
+    } else {
+      const int u0 = g0[cc], u1 = g0[n + m + cc];
+      const float4* Wg = reinterpret_cast<const float4*>(M.W + (int64_t)gi * D.w_size * K) + kq;
+      float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
+      if (u0 >= 0) x = __ldcg(Wg + ((int64_t)R.w0 + u0) * QC);
+      if (u1 >= 0) y = __ldcg(Wg + ((int64_t)R.w1 + u1) * QC);
+      sum.x += (float)((double)x.x + (double)y.x);
+      sum.y += (float)((double)x.y + (double)y.y);
+      sum.z += (float)((double)x.z + (double)y.z);
+      sum.w += (float)((double)x.w + (double)y.w);
+      *(reinterpret_cast<float4*>(M.W + ((int64_t)gi * D.w_size + R.woff + (cc - n)) * K) + kq) = sum;
+    }
+  }
+  if (pair + 2 * CB < r1) __syncthreads();  // the chains' space is free
+  }
+}
+
+// A task's factor rows are staged in what the vectors leave of the block's
+// shared memory, all at once where they fit, else in batches of row quads; the
+// first batch is in flight during the dependency wait and the gather.  Where not
+// even a quad fits (the largest fronts) the rows are read from L2.
+template <int K, bool TR>
+__global__ void __launch_bounds__(kMultiThreads, 2) k_multi(MultiDev M) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float4* V = reinterpret_cast<float4*>(smem_raw);
+  const ChainDev<float>& D = M.C;
+  __shared__ __align__(16) FlowClaim s_claims[2];  // the current task and the next
+  __shared__ int s_dep, s_o[K];
+  __shared__ SlotTables s_tab;
+  const int tid = threadIdx.x, lane = tid & 31;
+  build_slots(D, s_tab);
+  const uint64_t pol = stream_policy(false);
+  // The last warp claims the next task during the gather of the current one (a
+  // claim takes 1.7 us of a task's 12; every dependency is claimed earlier, so the
+  // earliest unfinished task is still the current one of its block).
+  const bool claimer = tid >= kMultiThreads - 32;
+  int slot = 0;
+  if (claimer) flow_claim(D, s_tab, s_claims[0], slot, K);
+  for (int cur = 0;; cur ^= 1) {
+    __syncthreads();
+    const FlowClaim& s_claim = s_claims[cur];
+    const int t = s_claim.t;
+    if (t >= D.total) break;
+    const FlowRec& R = s_claim.rec;
+    const int tau = TR ? (D.tau1 - 1 - s_claim.q) : (D.tau0 + s_claim.q);
+    const int gi = s_claim.gi, o0 = s_claim.o;
+    const int s = R.s, r0 = R.r0, r1 = R.r1, kind = R.kind_len & 255, n = R.n, m = R.m, ldn = R.ldn, ldm = R.ldm;
+    const int nk = min(K, D.Borb - gi * K);
+    if (tid >= 32 && tid < 32 + K) s_o[tid - 32] = D.orbit_ids[gi * K + (tid - 32 < nk ? tid - 32 : 0)];
+    int* cbase = D.counters + (int64_t)o0 * 8 * 2 * D.nsuper;  // the group's counters
+    const float* SQ = D.factors + ((int64_t)s_claim.set * D.n_bins + tau) * D.fac_size + R.fac_off;
+    const float* Qr = SQ + (int64_t)(n + m) * ldn;
+    // rows: shared positions of the vectors, and the stage behind them
+    const int at0 = kind == 0 ? 0 : r0 & ~3;
+    const int low = kind == 0 ? (min(r1, n) + 3) & ~3 : ((n + 3) & ~3) - at0;
+    const int own0 = max(r0, n);
+    const int positions = kind == 0 ? low + max(0, r1 - own0) : low + m;
+    float* stage = reinterpret_cast<float*>(V + (positions + 3) / 4 * K);
+    const int room = (M.smem_floats - (positions + 3) / 4 * 4 * K);
+    const int stride = TR ? 0 : (int)staged_row(kind, r0, r1, n, ldn, ldm);
+    const bool staged = !TR && room >= 4 * stride;
+    // rows a batch holds, its end on a quad boundary
+    auto batch_end = [&](int b0) { return staged ? min(r1, (b0 + room / max(stride, 4)) & ~3) : r1; };
+    auto stage_batch = [&](int b0, int b1) {
+      if (kind == 0) {
+        stage_rows<float, kMultiWarps>(stage, stride, SQ + (int64_t)b0 * ldn, ldn, b1 - b0, stride / 4, pol,
+                                       [](int) { return 0; }, [&](int r) { return (min(b0 + r, n) + 3) / 4; });
+      } else {
+        stage_rows<float, kMultiWarps>(stage, stride, SQ + (int64_t)b0 * ldn + at0, ldn, b1 - b0, (ldn - at0) / 4, pol,
+                                       [&](int r) { return (b0 + r - at0) / 4; },
+                                       [&](int) { return (n - at0 + 3) / 4; });
+        if (m > 0)
+          stage_rows<float, kMultiWarps>(stage + ldn - at0, stride, Qr + (int64_t)b0 * ldm, ldm, b1 - b0, ldm / 4, pol,
+                                         [](int) { return 0; }, [&](int) { return (m + 3) / 4; });
+      }
+    };
+    int b0 = r0, b1 = TR ? r0 : batch_end(r0);
+    if (staged) {
+      stage_batch(b0, b1);
+    } else if (!TR) {
+      const float* a = kind == 0 ? SQ + (int64_t)r0 * ldn : Qr + (int64_t)r0 * ldm;
+      const int64_t bytes = (int64_t)(r1 - r0) * (kind == 0 ? ldn : ldm) * (int64_t)sizeof(float);
+      for (int64_t b = (int64_t)tid * 128; b < bytes; b += (int64_t)kMultiThreads * 128)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(a) + b));
+    } else {
+      // ask L2 for the columns before waiting
+      const bool sq = kind == 3 || r0 < n;
+      const int ld = sq ? ldn : ldm;
+      const float* a = sq ? SQ + r0 : Qr + (r0 - n);
+      const int i0 = kind == 2 ? 0 : r0, i1 = kind == 3 ? n + m : sq ? min(r1, n) : n;
+      const int segs = (r1 - r0 + 31) / 32;
+      for (int b = tid; b < segs * (i1 - i0); b += kMultiThreads)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(a + (int64_t)(i0 + b / segs) * ld + min((b % segs) * 32, r1 - r0 - 1)));
+    }
+    if (tid < 32) {
+      // up to three counters, one lane each
+      const int* p = nullptr;
+      int want = 0;
+      if ((kind & 1) == 0) {
+        const int c = lane < 2 ? D.child[2 * s + lane] : -1;
+        const int prev = TR ? tau + 1 : tau - 1;
+        if (c >= 0) {
+          p = cbase + (tau * 2 + 0) * D.nsuper + c;
+          want = M.nch_f[c];
+        } else if (lane == 2 && (TR ? tau < D.tau1 - 1 : tau > D.tau0)) {
+          p = cbase + (prev * 2 + 1) * D.nsuper + s;
+          want = M.nch_b[s];
+        }
+      } else if (lane == 0) {
+        const int par = D.parent[s];
+        p = cbase + (par < 0 ? (tau * 2 + 0) * D.nsuper + s : (tau * 2 + 1) * D.nsuper + par);
+        want = par < 0 ? M.nch_f[s] : M.nch_b[par];
+      }
+      const bool ok = !p || wait_ge(p, want, D.status, D.spin_limit, D.spin_ns);
+      const bool all = __all_sync(0xffffffffu, ok);
+      if (lane == 0) s_dep = all;
+    }
+    __syncthreads();
+    if (!s_dep) {
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      break;
+    }
+    if (claimer) flow_claim(D, s_tab, s_claims[cur ^ 1], slot, K);
+    if (TR) {
+      if (r1 - r0 > 64) multi_cols<K, 2>(M, R, gi, s_o, nk, tau, SQ, V);
+      else multi_cols<K, 1>(M, R, gi, s_o, nk, tau, SQ, V);
+    } else {
+      if (kind == 0) {
+        multi_gather_fwd<K, false>(M, R, gi, s_o, tau, r0, r1, low, V);
+      } else {
+        const int32_t* ui = D.uidx + R.map_off;
+        multi_gather<K>(M.Y + ((int64_t)gi * D.N + R.first) * K, r0 - at0, n - r0, V, [&](int q2) { return r0 + q2; });
+        multi_gather<K>(M.X + (int64_t)gi * D.N * K, low, m, V, [&](int q2) { return ui[q2]; });
+      }
+      const int G = group_lanes<float>(R.kind_len >> 8);
+      const float* A0 = staged ? stage - at0 : SQ + (int64_t)r0 * ldn;
+      const float* B0 = staged ? stage + ldn - at0 : Qr + (int64_t)r0 * ldm;
+      const int lda = staged ? stride : ldn, ldb = staged ? stride : ldm;
+      for (;;) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        if (kind == 0) {
+          switch (G) {
+            case 4: multi_rows<4, K, true>(M, R, gi, s_o, nk, tau, b0, b1, A0, lda, B0, ldb, at0, low, own0, V); break;
+            case 8: multi_rows<8, K, true>(M, R, gi, s_o, nk, tau, b0, b1, A0, lda, B0, ldb, at0, low, own0, V); break;
+            case 16: multi_rows<16, K, true>(M, R, gi, s_o, nk, tau, b0, b1, A0, lda, B0, ldb, at0, low, own0, V); break;
+            default: multi_rows<32, K, true>(M, R, gi, s_o, nk, tau, b0, b1, A0, lda, B0, ldb, at0, low, own0, V); break;
+          }
+        } else {
+          switch (G) {
+            case 4: multi_rows<4, K, false>(M, R, gi, s_o, nk, tau, b0, b1, A0, lda, B0, ldb, at0, low, own0, V); break;
+            case 8: multi_rows<8, K, false>(M, R, gi, s_o, nk, tau, b0, b1, A0, lda, B0, ldb, at0, low, own0, V); break;
+            case 16: multi_rows<16, K, false>(M, R, gi, s_o, nk, tau, b0, b1, A0, lda, B0, ldb, at0, low, own0, V); break;
+            default: multi_rows<32, K, false>(M, R, gi, s_o, nk, tau, b0, b1, A0, lda, B0, ldb, at0, low, own0, V); break;
+          }
+        }
+        if (b1 >= r1) break;
+        __syncthreads();  // the stage is free
+        b0 = b1;
+        b1 = batch_end(b0);
+        stage_batch(b0, b1);
+      }
+    }
+    __syncthreads();
+    if (tid == 0) red_release_add(cbase + (tau * 2 + (kind & 1)) * D.nsuper + s, 1);
+  }
+}
+
 // x[tau0] += escale * E[tau0] (forcing of the transposed chain's last bin)
 __global__ void k_add_forcing(double* X, const double* E, const int* orbit_ids, int64_t N, int tau0,
                               double escale) {
@@ -1791,6 +2432,66 @@ bool chain_bound(const Symbolic& S, int B, size_t value_bytes) {
   return S.fac_nnz <= 30000000 && (double)B * (double)S.fac_nnz * (double)value_bytes <= 240e6;
 }
 
+// The FP32 many-right-hand-side kernels on a prepared launch: groups of K.
+int launch_multi(orbit_factor_s* f, const ChainDev<float>& C, int K, int ks, int B, int trans, double* X,
+                 const int* d_orbit_ids, int tau0, const double* E, double escale, int sms, cudaStream_t st) {
+  const Symbolic& S = f->sym->S;
+  MultiDev M;
+  M.C = C;
+  const int64_t groups = (B + K - 1) / K;
+  M.W = f->multi;
+  M.Y = M.W + groups * S.w_size * K;
+  M.X = M.Y + groups * S.N * K;
+  M.nch_f = C.nch_f;
+  M.nch_b = C.nch_b;
+  const FlowSched& P = trans ? S.wide : S.whole[ks];
+  const DevSym::Flow& p = trans ? f->sym->d.wide : f->sym->d.whole[ks];
+  M.C.recs = p.recs;
+  M.C.phase_off = p.phase_off;
+  M.C.items_per_bin = P.items_per_bin;
+  M.C.total = (C.tau1 - C.tau0) * P.items_per_bin * C.B;
+  if (trans) {
+    M.nch_f = f->sym->d.wide_nch_f;
+    M.nch_b = f->sym->d.wide_nch_b;
+  }
+  const void* fn = K == 16 ? (trans ? (const void*)k_multi<16, true> : (const void*)k_multi<16, false>)
+                   : K == 8 ? (trans ? (const void*)k_multi<8, true> : (const void*)k_multi<8, false>)
+                            : (trans ? (const void*)k_multi<4, true> : (const void*)k_multi<4, false>);
+  const size_t vectors = ((size_t)(trans ? S.max_nm : S.max_front) + 16) / 4 * 4 * K * sizeof(float);
+  // columns: the partial chains of two blocks of 64 columns
+  const size_t smem = std::max<size_t>(trans ? 3 * 4 * 64 * K * sizeof(float) : kMultiSmem, vectors);
+  M.smem_floats = (int)(smem / sizeof(float));
+  if (int r = allow_max_smem(fn)) return r;
+  int occ = 0;
+  ORBIT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kMultiThreads, smem));
+  if (occ < 1) {
+    set_last_error("chain kernel cannot be resident");
+    return ORBIT_ERR_INTERNAL;
+  }
+  const int grid = std::min(sms * occ, M.C.total);
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  if (f->prof_on) {
+    cudaEventCreate(&e0);
+    cudaEventCreate(&e1);
+    cudaEventRecord(e0, st);
+  }
+  void* args[] = {&M};
+  ORBIT_CUDA_TRY(cudaLaunchKernel(fn, dim3(grid), dim3(kMultiThreads), args, smem, st));
+  note_launch();
+  if (f->prof_on) {
+    cudaEventRecord(e1, st);
+    f->prof_chain.push_back({e0, e1});
+    f->prof_chain_bytes += (double)B * (C.tau1 - C.tau0) * S.fac_nnz * sizeof(float);
+  }
+  if (trans && E) {
+    dim3 g((unsigned)((S.N + 255) / 256), B);
+    k_add_forcing<<<g, 256, 0, st>>>(X, E, d_orbit_ids, S.N, tau0, escale);
+    note_launch();
+    ORBIT_CUDA_TRY(cudaGetLastError());
+  }
+  return ORBIT_OK;
+}
+
 template <typename T>
 int launch_chain_t(orbit_factor_s* f, double* X, int B, const int* d_orbit_ids, int trans, int tau0,
                    int tau1, const double* E, double escale, cudaStream_t st, bool never_ready = false) {
@@ -1802,9 +2503,13 @@ int launch_chain_t(orbit_factor_s* f, double* X, int B, const int* d_orbit_ids, 
   D.ginv = sy->d.ginv; D.ginv_off = sy->d.ginv_off;
   // Right-hand sides on one factor set go through the multi-RHS kernels in
   // groups of K (row-chunk tasks, forward and transposed sweeps).
-  constexpr int KM = sizeof(T) == 4 ? 4 : 2;
   const bool multi = !never_ready && f->n_sets == 1 && B >= 2 && S.max_sub_front == 0;
-  const int Bt = multi ? (B + KM - 1) / KM : B;  // task groups per (node chunk, bin)
+  constexpr int KM = 2;  // FP64 group size
+  // FP32 group size: the batch's, while its vectors leave a block resident
+  int KF = B > 8 ? 16 : B > 4 ? 8 : 4;
+  while (KF > 4 && (size_t)(S.max_front + 16) * KF * sizeof(float) > 215000) KF /= 2;
+  const int Kg = !multi ? 1 : sizeof(T) == 4 ? KF : KM;
+  const int Bt = (B + Kg - 1) / Kg;  // task groups per (node chunk, bin)
   // dataflow kernels: the transposed sweeps, and the others of launches bound
   // by their dependency chain
   const bool sub = S.max_sub_front > 0;
@@ -1814,9 +2519,12 @@ int launch_chain_t(orbit_factor_s* f, double* X, int B, const int* d_orbit_ids, 
   // transposed dataflow sweeps, whose sums do not depend on the chunks, go by
   // the factor entries that one bin's sweep of all groups reads instead (2 and
   // 6 groups of the 80x72x15 grid's 52 M).
+  // (The FP32 many-right-hand-side rows keep the schedule of groups of four,
+  // from which their lanes per row, and so the order of their sums, follow.)
+  const int Bs = multi && sizeof(T) == 4 ? (B + 3) / 4 : Bt;
   const int64_t bin_elems = (int64_t)Bt * S.fac_nnz;
   const int ks = flow && trans ? (bin_elems <= 110000000 && sizeof(T) == 8 ? 0 : bin_elems <= 330000000 ? 1 : 2)
-                               : (Bt <= 2 ? 0 : Bt <= 6 ? 1 : 2);
+                               : (Bs <= 2 ? 0 : Bs <= 6 ? 1 : 2);
   const bool rows = flow && !trans;
   const SolveSched& Q = S.sched[ks];
   const auto& q = sy->d.sched[ks];
@@ -1902,7 +2610,9 @@ int launch_chain_t(orbit_factor_s* f, double* X, int B, const int* d_orbit_ids, 
   int dev = 0, sms = 0, occ = 0;
   ORBIT_CUDA_TRY(cudaGetDevice(&dev));
   ORBIT_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  if (multi) {
+  if constexpr (sizeof(T) == 4)
+    if (multi) return launch_multi(f, D, KF, ks, B, trans, X, d_orbit_ids, tau0, E, escale, sms, st);
+  if constexpr (sizeof(T) == 8) if (multi) {
     const int vcap = (S.max_front + 8 + 3) & ~3;
     const size_t msmem = sizeof(T) * ((size_t)KM * vcap + (size_t)KM * kWarps * 32);
     {

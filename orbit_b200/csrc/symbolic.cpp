@@ -676,10 +676,38 @@ std::string build_symbolic(int nz, int ny, int nx, const SymbolicOptions& opt, S
     P.phase_off.push_back(int32_t(P.recs.size()));
     P.items_per_bin = P.phase_off.back();
   }
+  if (S.max_sub_front == 0) {
+    FlowSched& P = S.wide;
+    S.wide_nch_f.assign(ns, 0);
+    S.wide_nch_b.assign(ns, 0);
+    auto chunks = [&](int s, int kind) {
+      // cut at column n: 64 columns where they are long, else as many blocks of
+      // 128 as make a task of 32 K entries (forward tasks gather once for all)
+      const int n = S.n[s], cols = kind == 2 ? n + S.m[s] : n;
+      for (int c = 0; c < cols;) {
+        const int rows = kind == 2 ? n : n - c + S.m[s];
+        const int width = rows > 400 ? 64 : kind == 2 ? 128 * std::max(1, 256 / rows) : 128;
+        const int e = std::min(c + width, c < n ? n : cols);
+        P.recs.push_back(flow_rec(s, c, e, kind, 0));
+        ++(kind == 2 ? S.wide_nch_f : S.wide_nch_b)[s];
+        c = e;
+      }
+    };
+    for (int l = S.nlevels - 1; l >= 0; --l) {
+      P.phase_off.push_back(int32_t(P.recs.size()));
+      for (int s : S.level_sups[l]) chunks(s, 2);
+    }
+    for (int l = 0; l < S.nlevels; ++l) {
+      P.phase_off.push_back(int32_t(P.recs.size()));
+      for (int s : S.level_sups[l]) chunks(s, 3);
+    }
+    P.phase_off.push_back(int32_t(P.recs.size()));
+    P.items_per_bin = P.phase_off.back();
+  }
   for (int k = 0; k < kNumSched && S.max_sub_front == 0; ++k)
-    for (int prec = 0; prec < 2; ++prec) {
+    for (int prec = 0; prec < 3; ++prec) {  // FP32, FP64, uncut
       const SolveSched& Q = S.sched[k];
-      FlowSched& P = S.staged[k][prec];
+      FlowSched& P = prec < 2 ? S.staged[k][prec] : S.whole[k];
       const int64_t vb = prec ? 8 : 4;
       size_t ph = 0;
       for (int32_t i = 0; i < Q.items_per_bin; ++i) {
@@ -691,7 +719,7 @@ std::string build_symbolic(int nz, int ny, int nx, const SymbolicOptions& opt, S
         const int s = it[0], kind = it[3], n = S.n[s], m = S.m[s];
         const int len = kind == 0 ? std::min(it[2] - 1, n) : n - it[1] + m;
         for (int a = it[1]; a < it[2];) {
-          int b = a + 1;
+          int b = prec < 2 ? a + 1 : it[2];
           while (b < it[2]) {
             const int64_t full = (b + 1 - a) * staged_row(kind, a, b + 1, n, S.ldn[s], S.ldm[s]) * vb;
             if (full > kStageBytes || (full > kStageBytesCut && b - a >= 4)) break;

@@ -141,8 +141,13 @@ struct Symbolic {
   // and FP64 (1) factors.  A row keeps the lanes of its uncut chunk, and with
   // them the order of its sum.
   FlowSched staged[kNumSched][2];
+  FlowSched whole[kNumSched];  // and uncut
   // their transposed counterparts (column chunks, both precisions)
   FlowSched columns[kNumSched];
+  // column chunks of the many-right-hand-side transposed sweeps, and each
+  // supernode's number of them
+  FlowSched wide;
+  std::vector<int32_t> wide_nch_f, wide_nch_b;
   std::vector<int32_t> role;  // 0 chunked node, 1 subtree-task root, 2 inside a subtree
   int max_front = 0;
   int max_sub_front = 0;  // largest n+m of a supernode inside a subtree task

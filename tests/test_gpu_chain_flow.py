@@ -1,4 +1,5 @@
-"""Chained sweeps of small domains (B200): the dataflow kernels.
+"""Chained sweeps (B200): the dataflow kernels of small domains, and the
+kernels of many right-hand sides on one factor set.
 
 Sweeps of domains too small to fill the GPU run on kernels that hand tagged
 values from task to task, with the factor rows staged in shared memory, and
@@ -18,10 +19,15 @@ EPS = {64: 2.0 ** -53, 32: 2.0 ** -24}
 
 
 @pytest.mark.parametrize("precision", [64, 32])
-@pytest.mark.parametrize("shape,leaf,batch,periodic", [
-    ((3, 4, 5), 4, 1, False), ((5, 7, 6), 16, 3, False), ((7, 11, 13), 8, 2, False), ((6, 17, 19), 40, 5, False),
-    ((9, 23, 29), 64, 1, False), ((5, 9, 16), 24, 2, True), ((2, 2, 3), 1, 1, False)])
-def test_sweeps_match_sparse_solves(shape, leaf, batch, periodic, precision):
+@pytest.mark.parametrize("shape,leaf,batch,sets,periodic", [
+    ((3, 4, 5), 4, 1, 1, False), ((5, 7, 6), 16, 3, 2, False), ((7, 11, 13), 8, 2, 2, False),
+    ((6, 17, 19), 40, 5, 2, False), ((9, 23, 29), 64, 1, 1, False), ((5, 9, 16), 24, 2, 2, True),
+    ((2, 2, 3), 1, 1, 1, False),
+    # groups of 4, 8 and 16 right-hand sides, whole and not
+    ((5, 7, 6), 16, 2, 1, False), ((2, 2, 3), 1, 4, 1, False), ((7, 11, 13), 8, 5, 1, False),
+    ((5, 9, 16), 24, 8, 1, True), ((9, 23, 29), 64, 9, 1, False), ((8, 21, 26), 100, 17, 1, False),
+    ((6, 17, 19), 40, 33, 1, False)])
+def test_sweeps_match_sparse_solves(shape, leaf, batch, sets, periodic, precision):
     import scipy.sparse as sp
     import scipy.sparse.linalg as spl
     import torch
@@ -31,7 +37,6 @@ def test_sweeps_match_sparse_solves(shape, leaf, batch, periodic, precision):
     met = synthetic.make_met(5, nz, ny, nx, cmfmc_frac=0.3, periodic=periodic)
     mets = [device.MetDevice(g) for g in met]
     T = [device.assemble_transport(m) for m in mets]
-    sets = min(batch, 2)
     d = [synthetic.make_species(6 + q, nz, ny, nx).sink_diag(met) for q in range(sets)]
     sym = Symbolic(nz, ny, nx, leaf, periodic=periodic)
     fb = device.FactorBatch(sym, batch, precision, n_sets=sets)
