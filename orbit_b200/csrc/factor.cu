@@ -447,7 +447,7 @@ __device__ __forceinline__ void gemm_tile(const T* __restrict__ A, int lda, cons
 // elements, its columns may start anywhere), zero-filled beyond h, w and K.
 // Row strides of 20 and 68 doubles put a half-warp's fragment reads in distinct
 // banks.  Measured on the 80x72x15 grid, 8 bins, one species: Schur complements
-// 17.3 -> 9.4 ms (11.2 with C read after the products), trailing updates 9.3 -> 5.6, panel products 8.9 -> 4.7.
+// 17.3 -> 9.3 ms (11.2 without the prefetch of C), trailing updates 9.3 -> 5.3, panel products 8.9 -> 4.8.
 constexpr int kDmK = 16, kDmLdA = kDmK + 4, kDmLdB = 64 + 4, kDmStages = 3;
 constexpr int kDmStage = 128 * kDmLdA + kDmK * kDmLdB;  // doubles
 
@@ -488,20 +488,22 @@ __device__ __forceinline__ void gemm_dmma(const double* __restrict__ A, int lda,
     if (s < slabs) load(s);
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
-  // the accumulators start from C (read while the first slabs are on their way)
-  // and take -A B; warps whose outputs all lie outside the tile only help with
-  // the copies
+  // warps whose outputs all lie outside the tile only help with the copies;
+  // the others ask L2 for the outputs that they update.  (The sums do not start
+  // from C: each step would then round at C's magnitude.)
   const bool on = wr < h && wc < w;
+  if (!assign && on)
+    for (int q = lane; q < 96; q += 32) {
+      const int r = wr + q / 3, c = min(wc + 16 * (q % 3), w - 1);
+      if (r < h && c < wc + 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(C + (int64_t)r * ldc + c));
+    }
   double acc[2][4][4];
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int r = wr + 16 * i + 8 * (q >> 1) + g, c = wc + 8 * j + 2 * t + (q & 1);
-        acc[i][j][q] = !assign && r < h && c < w ? C[(int64_t)r * ldc + c] : 0.0;
-      }
+      for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.0;
   for (int s = 0; s < slabs; ++s) {
     asm volatile("cp.async.wait_group %0;" ::"n"(kDmStages - 2) : "memory");
     __syncthreads();
@@ -515,10 +517,10 @@ __device__ __forceinline__ void gemm_dmma(const double* __restrict__ A, int lda,
       double a[2][4], b[4][2];
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        a[i][0] = -As[(16 * i) * kDmLdA + kk];
-        a[i][1] = -As[(16 * i + 8) * kDmLdA + kk];
-        a[i][2] = -As[(16 * i) * kDmLdA + kk + 4];
-        a[i][3] = -As[(16 * i + 8) * kDmLdA + kk + 4];
+        a[i][0] = As[(16 * i) * kDmLdA + kk];
+        a[i][1] = As[(16 * i + 8) * kDmLdA + kk];
+        a[i][2] = As[(16 * i) * kDmLdA + kk + 4];
+        a[i][3] = As[(16 * i + 8) * kDmLdA + kk + 4];
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -534,15 +536,37 @@ __device__ __forceinline__ void gemm_dmma(const double* __restrict__ A, int lda,
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
   if (!on) return;
+  if (assign) {
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int r = wr + 16 * i + 8 * (q >> 1) + g, c = wc + 8 * j + 2 * t + (q & 1);
+          if (r < h && c < w && !(r >= skip_r && c >= skip_c)) C[(int64_t)r * ldc + c] = -acc[i][j][q];
+        }
+    return;
+  }
+  // all of a row block's outputs read before the first is written
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    double v[4][4];
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const int r = wr + 16 * i + 8 * (q >> 1) + g, c = wc + 8 * j + 2 * t + (q & 1);
-        if (r < h && c < w && !(r >= skip_r && c >= skip_c)) C[(int64_t)r * ldc + c] = acc[i][j][q];
+        v[j][q] = r < h && c < w ? C[(int64_t)r * ldc + c] : 0.0;
       }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int r = wr + 16 * i + 8 * (q >> 1) + g, c = wc + 8 * j + 2 * t + (q & 1);
+        if (r < h && c < w && !(r >= skip_r && c >= skip_c)) C[(int64_t)r * ldc + c] = v[j][q] - acc[i][j][q];
+      }
+  }
 }
 
 // C tile (128 x 128) -= / = - A B with K in [k0, K): FP32 as one 128x128
