@@ -324,9 +324,10 @@ int orbit_stencil_apply_grid(int nz, int ny, int nx, int periodic_x, int n_vec, 
  * owns its whole device-memory budget through its own pool, or a time loop
  * that must not stall on the synchronization cudaFree can cause).  Same inputs,
  * outputs and results as orbit_fct_source.  No counterpart in the reference.
- * The scratch (x = c/rho, R+, R-) is one static device array of 3 x 2^20
- * doubles (24 MiB) that every GPU loading this library holds until exit, so
- * n_vec*nz*ny*nx must be <= 1,048,576 (larger requests return ORBIT_ERR_ARG).
+ * The scratch (a copy of c, made where d overlaps it) is one static device
+ * array of 2^20 doubles (8 MiB) that every GPU loading this library holds until
+ * exit, so n_vec*nz*ny*nx must be <= 1,048,576 (larger requests return
+ * ORBIT_ERR_ARG).
  * The first call on a device looks up the array's device address; make that
  * first call before any stream capture.  The address is cached per device
  * ordinal for the life of the process and does not survive a cudaDeviceReset

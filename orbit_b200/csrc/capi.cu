@@ -51,8 +51,9 @@ int assemble_transport(int nz, int ny, int nx, const orbit_met_t* met, double* T
 int chain_wait_selftest(orbit_factor_s* f, const int* d_orbit_ids, cudaStream_t st);
 int mass_balance_rows(int nz, int ny, int nx, int nbins, const double* const* Tst,
                       const double* const* rho, double* out_int, double* out_top, cudaStream_t st);
+bool fct_overlaps(const double* c, const double* d, int64_t n);
 int fct_source(int nz, int ny, int nx, const orbit_met_t* met, int n_vec, const double* c, double dt,
-               int limited, double* d, double* scratch, cudaStream_t st, const double* ghost = nullptr);
+               int limited, double* d, cudaStream_t st, const double* ghost = nullptr);
 int fct_source_noalloc(int nz, int ny, int nx, const orbit_met_t* met, int n_vec, const double* c,
                        double dt, int limited, double* d, cudaStream_t st);
 int fct_linear_operator(int nz, int ny, int nx, const orbit_met_t* met, int n_vec, const double* c, double dt,
@@ -156,6 +157,19 @@ int build_device_symbolic(orbit_symbolic_s* h) {
   ORBIT_TRY(upload(A, &d.ginv, S.ginv));
   ORBIT_TRY(upload(A, &d.ginv_off, S.ginv_off));
   return ORBIT_OK;
+}
+
+// The FCT source; a c that overlaps d is copied first.
+int fct_source_any(int nz, int ny, int nx, const orbit_met_t* met, int n_vec, const double* c, const double* ghost,
+                   double dt, int limited, double* d, cudaStream_t st) {
+  const int64_t n = (int64_t)nz * ny * nx * n_vec;
+  if (!fct_overlaps(c, d, n)) return fct_source(nz, ny, nx, met, n_vec, c, dt, limited, d, st, ghost);
+  double* copy = nullptr;
+  ORBIT_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&copy), sizeof(double) * n, st));
+  cudaError_t e = cudaMemcpyAsync(copy, c, sizeof(double) * n, cudaMemcpyDeviceToDevice, st);
+  int rc = e == cudaSuccess ? fct_source(nz, ny, nx, met, n_vec, copy, dt, limited, d, st, ghost) : ORBIT_ERR_CUDA;
+  cudaFreeAsync(copy, st);
+  return rc;
 }
 
 constexpr int kDefaultLeaf = 64;
@@ -404,13 +418,7 @@ int orbit_fct_source(int nz, int ny, int nx, const orbit_met_t* met, int n_vec, 
     set_last_error("orbit_fct_source: bad arguments");
     return ORBIT_ERR_ARG;
   }
-  cudaStream_t st = (cudaStream_t)stream;
-  const int64_t N = (int64_t)nz * ny * nx;
-  double* scratch = nullptr;
-  ORBIT_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&scratch), sizeof(double) * 3 * N * n_vec, st));
-  int rc = fct_source(nz, ny, nx, met, n_vec, c, dt, limited, d, scratch, st);
-  cudaFreeAsync(scratch, st);
-  return rc;
+  return fct_source_any(nz, ny, nx, met, n_vec, c, nullptr, dt, limited, d, (cudaStream_t)stream);
 }
 
 int orbit_fct_linear_operator(int nz, int ny, int nx, const orbit_met_t* met, int n_vec, const double* c_base,
@@ -434,13 +442,7 @@ int orbit_fct_source_ghost(int nz, int ny, int nx, const orbit_met_t* met, int n
     set_last_error("orbit_fct_source_ghost: bad arguments");
     return ORBIT_ERR_ARG;
   }
-  cudaStream_t st = (cudaStream_t)stream;
-  const int64_t N = (int64_t)nz * ny * nx;
-  double* scratch = nullptr;
-  ORBIT_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&scratch), sizeof(double) * 3 * N * n_vec, st));
-  int rc = fct_source(nz, ny, nx, met, n_vec, c, dt, limited, d, scratch, st, c_ghost);
-  cudaFreeAsync(scratch, st);
-  return rc;
+  return fct_source_any(nz, ny, nx, met, n_vec, c, c_ghost, dt, limited, d, (cudaStream_t)stream);
 }
 
 int orbit_stencil_apply(int nz, int ny, int nx, int n_vec, const double* stencils, const double* x, double alpha,
