@@ -40,16 +40,16 @@ namespace {
 #ifndef ORBIT_SOLVE_THREADS
 #define ORBIT_SOLVE_THREADS 128
 #endif
-// CTAs per SM the chain kernels are compiled for, per precision: FP32 at 10
-// (48 registers) hides more of the per-task latency than at 8 (64 registers),
-// 4 % faster on a 12-orbit chain even with the few spills it costs; FP64 at 7
-// (72 registers), which holds twelve 16-byte loads per lane in flight
-#ifndef ORBIT_SOLVE_MINB
-#define ORBIT_SOLVE_MINB 7
-#endif
-#ifndef ORBIT_SOLVE_MINB_FP32
-#define ORBIT_SOLVE_MINB_FP32 10
-#endif
+// Blocks per SM the counter kernels are compiled for, per precision: many hide
+// more of the per-task latency of launches that fill the GPU (FP32 10 with 48
+// registers, FP64 7 with 72), fewer leave registers for the loads in flight of
+// the others.  FP32, 80x72x15 grid, 8 bins, 1 / 4 / 12 orbits at 10 and at 8
+// blocks: 1.55 / 2.74 / 6.03 and 1.39 / 2.62 / 6.25 ms, 60x54x15 with 12 orbits 3.77
+// and 3.41; FP64, 1 / 2 / 4 orbits at 7 and at 6: 1.81 / 2.65 / 4.00 and 1.73 /
+// 2.73 / 4.11, 60x54x15 with 4 orbits 2.47 and 2.35.  So the line lies between the
+// factor bytes of one bin of all orbits in those launches.
+constexpr int kChainBlocks[2] = {10, 7}, kChainBlocksFew[2] = {8, 6};  // FP32, FP64
+constexpr double kChainManyBytes[2] = {1.6e9, 0.6e9};
 constexpr int kSolveThreads = ORBIT_SOLVE_THREADS;
 constexpr int kMaxPhases = 96;  // 2 x tree levels
 constexpr int kWarps = kSolveThreads / 32;
@@ -213,16 +213,17 @@ __device__ __forceinline__ double dot16(const double2& a, const double* v) {
 }
 
 // 16-byte loads in flight per lane in the row dot products of the chained
-// solves, per precision.  Measured on the 80x72x15 grid (8 bins, CUDA events):
-// FP32, 12 orbits at 10 CTAs per SM: 7.21 ms at 4, 6.94 at 6, 7.05 at 7 (8 at
-// 8 CTAs per SM: 7.55); FP64 at 7 CTAs per SM, 1 / 12 orbits: 1.76 / 9.83 ms
-// at 12 (2.44 ms / - at 4 and 8 CTAs per SM; 1.81 / 10.9 at 10; 1.81 / 11.1
-// at 16 and 6 CTAs per SM).
+// solves, per precision.  FP32 6 (7.21 ms at 4, 6.94 at 6, 7.05 at 7 for the
+// 12-orbit chain when it was chosen; a row's lanes, and with them the order of
+// its sum, follow from it).  FP64 8: with the rows' ends in the first round, 6 / 8
+// / 10 / 12 give 1.73 / 1.73 / 1.88 / 1.93 ms for one orbit of the 80x72x15 grid at
+// 6 to 7 blocks per SM (10 and 12 spill), 2.63 / 2.35 / 2.62 / 2.77 for four of the
+// 60x54x15 grid.
 #ifndef ORBIT_SOLVE_DEPTH_FP32
 #define ORBIT_SOLVE_DEPTH_FP32 6
 #endif
 #ifndef ORBIT_SOLVE_DEPTH_FP64
-#define ORBIT_SOLVE_DEPTH_FP64 12
+#define ORBIT_SOLVE_DEPTH_FP64 8
 #endif
 template <typename T> struct Depth { static constexpr int value = sizeof(T) == 4 ? ORBIT_SOLVE_DEPTH_FP32 : ORBIT_SOLVE_DEPTH_FP64; };
 
@@ -283,27 +284,37 @@ struct SharedRow {
 
 // Per-lane partial of sum_{j0 <= j < j1} a[j] v[j] for a group of G lanes
 // (gl = lane within the group; a 16-byte aligned at j = 0, v in shared memory,
-// 16-byte aligned).  16-byte loads, up to U in flight per lane: the unrolled
-// loop issues its guarded loads before it uses any of them.
+// 16-byte aligned).  16-byte loads, up to U in flight per lane, the guarded loads
+// of a round issued before any of them is used.  The unaligned ends (fewer than
+// 4 elements, so at most one per lane) are read together with the first round:
+// one memory latency for a row of up to U G vectors, where the ends used to cost
+// one each (8 bins, ms: FP32, 12 orbits, 80x72x15 6.55 -> 6.03, 60x54x15 4.55 -> 3.77; one orbit of the
+// 24x20x15 grid from shared memory 0.51 -> 0.45).
 template <typename T, int G = 32, int U = Depth<T>::value, typename Row = GlobalRow>
 __device__ __forceinline__ T dot_seg(const T* __restrict__ a, const T* v, int j0, int j1, int gl, const Row& row) {
   using V = typename Vec16<T>::type;
   constexpr int W = Vec16<T>::w;
+  static_assert(G >= W, "one end element per lane");
   T acc0 = T(0), acc1 = T(0), acc2 = T(0), acc3 = T(0);
   // [j0, ja) scalar head up to the first aligned index, [ja, jb) 16-byte
   // vectors, [jb, j1) scalar tail
   const int ja = min((j0 + W - 1) / W * W, j1);
   const int jb = max(ja, j1 / W * W);
-  for (int j = j0 + gl; j < ja; j += G) acc0 = fma(row.one(a + j), v[j], acc0);
-  const int nv0 = ja / W, nv1 = jb / W;
+  const int nv1 = jb / W;
   const V* a4 = reinterpret_cast<const V*>(a);
-  for (int k = nv0 + gl; k < nv1; k += U * G) {
-    V x[U];
+  const bool head = j0 + gl < ja, tail = jb + gl < j1;
+  T h = T(0), t = T(0);
+  if (head) h = row.one(a + j0 + gl);
+  if (tail) t = row.one(a + jb + gl);
+  int k = ja / W + gl;
+  V x[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      x[u] = V{};
-      if (u == 0 || k + u * G < nv1) x[u] = row.vec(a4 + k + u * G);
-    }
+  for (int u = 0; u < U; ++u) {
+    x[u] = V{};
+    if (k + u * G < nv1) x[u] = row.vec(a4 + k + u * G);
+  }
+  if (head) acc0 = fma(h, v[j0 + gl], acc0);
+  while (k < nv1) {
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if (u == 0 || k + u * G < nv1) {
@@ -313,8 +324,16 @@ __device__ __forceinline__ T dot_seg(const T* __restrict__ a, const T* v, int j0
         else if ((u & 3) == 2) acc2 += d;
         else acc3 += d;
       }
+    k += U * G;
+    if (k < nv1) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        x[u] = V{};
+        if (u == 0 || k + u * G < nv1) x[u] = row.vec(a4 + k + u * G);
+      }
+    }
   }
-  for (int j = jb + gl; j < j1; j += G) acc1 = fma(row.one(a + j), v[j], acc1);
+  if (tail) acc1 = fma(t, v[jb + gl], acc1);
   return (acc0 + acc1) + (acc2 + acc3);
 }
 
@@ -647,9 +666,9 @@ __device__ void bwd_node_warp(const ChainDev<T>& D, int o, int tau, int s, bool 
 
 // One instantiation per sweep direction (TR: transposed) and per schedule
 // kind (SUB: the schedule has whole-subtree tasks), so that each kernel
-// carries only the code its tasks run.
-template <typename T, bool TR, bool SUB>
-__global__ void __launch_bounds__(kSolveThreads, sizeof(T) == 4 ? ORBIT_SOLVE_MINB_FP32 : ORBIT_SOLVE_MINB) k_chain(ChainDev<T> D) {
+// carries only the code its tasks run; FEW: fewer blocks per SM.
+template <typename T, bool TR, bool SUB, bool FEW>
+__global__ void __launch_bounds__(kSolveThreads, (FEW ? kChainBlocksFew : kChainBlocks)[sizeof(T) == 8]) k_chain(ChainDev<T> D) {
   extern __shared__ unsigned char smem_raw[];
   T* red = reinterpret_cast<T*>(smem_raw);      // kWarps * 32
   T* vec = red + kWarps * 32;                    // front-sized vector
@@ -1484,7 +1503,7 @@ __device__ __forceinline__ void grouped_rows_multi(int r0, int r1, int wid, int 
   } while (0)
 
 template <typename T, int K>
-__global__ void __launch_bounds__(kSolveThreads, sizeof(T) == 4 ? ORBIT_SOLVE_MINB_FP32 : ORBIT_SOLVE_MINB) k_chain_multi(ChainDev<T> D, int vcap) {
+__global__ void __launch_bounds__(kSolveThreads, kChainBlocks[sizeof(T) == 8]) k_chain_multi(ChainDev<T> D, int vcap) {
   extern __shared__ unsigned char smem_raw[];
   T* vbuf = reinterpret_cast<T*>(smem_raw);  // K vectors of vcap
   T* red = vbuf + (int64_t)K * vcap;          // K x kWarps x 32 (transposed sweeps)
@@ -2421,15 +2440,15 @@ unsigned chain_spin_ns() {
 }
 
 // Whether a launch of B groups is bound by its dependency chain rather than by
-// the factor values it reads: on domains of up to 30 M factor entries per bin,
-// while one bin of all groups holds at most 240 MB.  Staged against direct
-// kernel, 8 bins, ms: 24x20x15 FP64 1 orbit 0.51 / 0.99, FP32 24 orbits (207 MB)
-// 1.6 / 2.3; 53x47x13 FP64 2 orbits (237 MB) 1.45 / 1.55, FP32 4 (237 MB)
-// 1.72 / 2.14; 60x54x15 FP64 1 orbit (210 MB) 1.32 / 1.49, FP32 4 (420 MB)
-// 2.9 / 2.4; 40x36x15 FP32 12 (440 MB) 3.04 / 3.00; 80x72x15 (52 M entries) FP64
-// 1 orbit 2.4 / 1.8.
-bool chain_bound(const Symbolic& S, int B, size_t value_bytes) {
-  return S.fac_nnz <= 30000000 && (double)B * (double)S.fac_nnz * (double)value_bytes <= 240e6;
+// the factor values it reads: up to 40 M factor entries per bin of all groups,
+// 60 M where a group's tree is small (its chunks are few).  k_flow against
+// k_chain, 8 bins, ms: 24x20x15 FP64 1 orbit 0.45 / 0.96, FP32 24 orbits (52 M) 1.54
+// / 1.76; 40x36x15 FP64 4 orbits (37 M) 1.65 / 1.74, FP32 4 1.09 / 1.41; 53x47x13
+// FP64 2 orbits (30 M) 1.32 / 1.40, FP32 4 (59 M) 1.64 / 1.56; 60x54x15 FP64 1 orbit
+// (26 M) 1.27 / 1.35, FP32 2 (53 M) 1.68 / 1.32; 80x72x15 FP64 1 orbit (52 M) 2.4 /
+// 1.7.
+bool chain_bound(const Symbolic& S, int B) {
+  return (int64_t)B * S.fac_nnz <= (S.fac_nnz <= 5000000 ? 60000000 : 40000000);
 }
 
 // The FP32 many-right-hand-side kernels on a prepared launch: groups of K.
@@ -2513,7 +2532,7 @@ int launch_chain_t(orbit_factor_s* f, double* X, int B, const int* d_orbit_ids, 
   // dataflow kernels: the transposed sweeps, and the others of launches bound
   // by their dependency chain
   const bool sub = S.max_sub_front > 0;
-  const bool flow = !multi && !sub && (trans || never_ready || chain_bound(S, Bt, sizeof(T)));
+  const bool flow = !multi && !sub && (trans || never_ready || chain_bound(S, Bt));
   // Schedule by batch size: small chunks shorten one orbit's critical path,
   // large ones cut per-task overhead when many orbits fill the GPU.  The
   // transposed dataflow sweeps, whose sums do not depend on the chunks, go by
@@ -2598,11 +2617,12 @@ int launch_chain_t(orbit_factor_s* f, double* X, int B, const int* d_orbit_ids, 
       rows ? kStageBytes + sizeof(T) * ((size_t)S.max_front + 8)
            : sizeof(T) * ((size_t)kWarps * 32 * (flow && sizeof(T) == 4 ? 4 : 1) +
                           std::max<size_t>(S.max_front + 8, (size_t)kWarps * ((S.max_sub_front + 7) & ~3)) + 8);
+  const bool few = (double)bin_elems * sizeof(T) <= kChainManyBytes[sizeof(T) == 8];
   const void* kfn = rows    ? (const void*)k_flow<T>
                     : flow  ? (const void*)k_flow_t<T>
-                    : !sub  ? (const void*)k_chain<T, false, false>
-                    : trans ? (const void*)k_chain<T, true, true>
-                            : (const void*)k_chain<T, false, true>;
+                    : !sub  ? (few ? (const void*)k_chain<T, false, false, true> : (const void*)k_chain<T, false, false, false>)
+                    : trans ? (const void*)k_chain<T, true, true, false>
+                            : (const void*)k_chain<T, false, true, false>;
   {
     int r0 = allow_max_smem(kfn);
     if (r0) return r0;
@@ -2663,9 +2683,10 @@ int launch_chain_t(orbit_factor_s* f, double* X, int B, const int* d_orbit_ids, 
   }
   if (rows) k_flow<T><<<grid, kSolveThreads, smem, st>>>(D);
   else if (flow) k_flow_t<T><<<grid, kSolveThreads, smem, st>>>(D);
-  else if (!sub) k_chain<T, false, false><<<grid, kSolveThreads, smem, st>>>(D);
-  else if (trans) k_chain<T, true, true><<<grid, kSolveThreads, smem, st>>>(D);
-  else k_chain<T, false, true><<<grid, kSolveThreads, smem, st>>>(D);
+  else if (!sub && few) k_chain<T, false, false, true><<<grid, kSolveThreads, smem, st>>>(D);
+  else if (!sub) k_chain<T, false, false, false><<<grid, kSolveThreads, smem, st>>>(D);
+  else if (trans) k_chain<T, true, true, false><<<grid, kSolveThreads, smem, st>>>(D);
+  else k_chain<T, false, true, false><<<grid, kSolveThreads, smem, st>>>(D);
   note_launch();
   if (f->prof_on) {
     cudaEventRecord(e1, st);
