@@ -503,12 +503,35 @@ int matvec(Ctx& c, const double* v, int64_t vstride, double* w, int64_t wstride,
   return ORBIT_OK;
 }
 
+// V0 = s - (I - M) x by one sweep from x with the forcing F whose sweep from
+// zero is s: it ends at M x + s, and leaves the orbit that x stands for in f->X
+// (transposed: the receptors of bins 1..7 not yet added).
+int forced_residual(Ctx& c, const double* F, double fscale, const double* x, double* V0, int64_t vstr,
+                    const int* d_ids, int B) {
+  orbit_factor_s* f = c.f;
+  const int64_t N = c.N;
+  const dim3 g = vgrid(N, B);
+  Scal one{nullptr, 0, 0, 1.0}, mone{nullptr, 0, 0, -1.0};
+  const int in = c.trans ? 8 : 0, out = c.trans ? 0 : 8;
+  k_lincomb<<<g, kVT, 0, c.st>>>(f->X + in * N, 9 * N, one, x, c.vs, one, nullptr, 0, d_ids, N);
+  note_launch();
+  int rc = launch_chain(f, B, d_ids, c.trans, 0, 8, F, fscale, c.st);
+  if (rc) return rc;
+  k_lincomb<<<g, kVT, 0, c.st>>>(V0, vstr, one, f->X + out * N, 9 * N, mone, x, c.vs, d_ids, N);
+  note_launch();
+  ORBIT_CUDA_TRY(cudaGetLastError());
+  return ORBIT_OK;
+}
+
 // Restarted GMRES on (I - M) x = b for the orbits in `act`; x, b per orbit (stride vs).
+// With F (FP64 solves; b = the sweep of F from zero) the residuals come from sweeps
+// with that forcing, the last of which is the orbit's recovery sweep: a solve takes
+// one sweep fewer.
 // atol per orbit; iters accumulated; converged flags set.  rn_out gets the final true residual norm.
 int gmres(Ctx& c, std::vector<int> act, double* b, double* x, const std::vector<double>& atol,
           int maxiter, bool accurate_mv, std::vector<int>& iters, std::vector<int>& conv,
           std::vector<double>& rn_out, std::vector<int>& matvecs, bool x_is_zero,
-          bool trust_estimate = false) {
+          bool trust_estimate = false, const double* F = nullptr, double fscale = 0.0) {
   orbit_factor_s* f = c.f;
   const int64_t N = c.N;
   const int R = c.R;
@@ -527,6 +550,10 @@ int gmres(Ctx& c, std::vector<int> act, double* b, double* x, const std::vector<
   if (x_is_zero) {
     k_lincomb<<<vgrid(N, B), kVT, 0, c.st>>>(V_of(0), vstr, one, b, c.vs, one, nullptr, 0, d_ids, N);
     note_launch();
+  } else if (F) {
+    rc = forced_residual(c, F, fscale, x, V_of(0), vstr, d_ids, B);
+    if (rc) return rc;
+    for (int o : act) matvecs[o]++;
   } else {
     rc = matvec(c, x, c.vs, c.Rv, c.vs, d_ids, B, accurate_mv);
     if (rc) return rc;
@@ -640,11 +667,16 @@ int gmres(Ctx& c, std::vector<int> act, double* b, double* x, const std::vector<
       if (rc) return rc;
     }
     // true residual r = b - A x -> V0 (unnormalised) and its norm
-    rc = matvec(c, x, c.vs, c.Rv, c.vs, d_ids, B, accurate_mv);
-    if (rc) return rc;
+    if (F) {
+      rc = forced_residual(c, F, fscale, x, V_of(0), vstr, d_ids, B);
+      if (rc) return rc;
+    } else {
+      rc = matvec(c, x, c.vs, c.Rv, c.vs, d_ids, B, accurate_mv);
+      if (rc) return rc;
+      k_lincomb<<<vgrid(N, B), kVT, 0, c.st>>>(V_of(0), vstr, one, b, c.vs, mone, c.Rv, c.vs, d_ids, N);
+      note_launch();
+    }
     for (int o : act) matvecs[o]++;
-    k_lincomb<<<vgrid(N, B), kVT, 0, c.st>>>(V_of(0), vstr, one, b, c.vs, mone, c.Rv, c.vs, d_ids, N);
-    note_launch();
     rc = sqnorm(c, V_of(0), vstr, d_ids, B, S_NORM);
     if (rc) return rc;
     rc = fetch_scal(c);
@@ -690,7 +722,7 @@ int orbit_solve_impl(orbit_factor_s* f, int n, const double* e_or_R, double dtau
   note_launch();
   // s: forward x0 = 0, P_tau(x + dtau e); adjoint x8 = 0, P^T x + R
   Scal one{nullptr, 0, 0, 1.0}, zero{nullptr, 0, 0, 0.0};
-  const int in = trans ? 8 : 0, outb = trans ? 0 : 8;
+  const int outb = trans ? 0 : 8;
   ORBIT_CUDA_TRY(cudaMemsetAsync(f->X, 0, sizeof(double) * 9 * N * n, st));
   const double fscale = trans ? 1.0 : dtau;
   std::vector<int> mv(f->n_orbits, 0), iters(f->n_orbits, 0), conv(f->n_orbits, 0), outer(f->n_orbits, 0);
@@ -731,7 +763,7 @@ int orbit_solve_impl(orbit_factor_s* f, int n, const double* e_or_R, double dtau
   }
   bool mixed_done = false;
   if (!c.mixed) {
-    rc = gmres(c, act, c.Sv, c.Xv, atol, maxiter, false, iters, conv, rn, mv, false);
+    rc = gmres(c, act, c.Sv, c.Xv, atol, maxiter, false, iters, conv, rn, mv, false, false, f->E, fscale);
     if (rc) return rc;
   } else if (!trans) {
     // Block-cyclic FP64 refinement.  The orbit is the solution of the eight
@@ -954,44 +986,28 @@ int orbit_solve_impl(orbit_factor_s* f, int n, const double* e_or_R, double dtau
     note_launch();
     mixed_done = true;
   }
-  // recovery: chain with forcing from x
   rc = upload_ids(c, all, d_ids);
   if (rc) return rc;
   if (!mixed_done) {
-  ORBIT_CUDA_TRY(cudaMemsetAsync(f->X, 0, sizeof(double) * 9 * N * n, st));
-  k_lincomb<<<g, kVT, 0, st>>>(f->X + in * N, 9 * N, one, c.Xv, c.vs, zero, nullptr, 0, d_ids, N);
-  note_launch();
-  if (!trans) {
-    rc = chain_accurate(c, d_ids, n, f->E, fscale);
-    if (rc) return rc;
-  } else {
-    // adjoint unroll: lam_tau = P_tau^T lam_{tau+1} + R_tau for tau = 7..1, lam_8 = lam_0
-    rc = chain_accurate(c, d_ids, n, f->E, fscale, 1, 8);
-    if (rc) return rc;
-    // X[tau] for tau = 2..7 hold P^T(...) without R: add R_tau (X[1] already has it)
-    for (int t = 2; t < 8; ++t) {
-      k_lincomb<<<g, kVT, 0, st>>>(f->X + t * N, 9 * N, one, f->X + t * N, 9 * N, one, f->E + t * N, 8 * N, d_ids, N);
+    // The last residual sweep of every orbit started from its solution x, with
+    // the forcing: f->X holds the recovered orbit (an orbit of zero forcing has
+    // zeros there), and its end against x is the periodicity, forward
+    // ||X8 - X0|| / (||X0|| + 1e-30), adjoint ||P_0^T lam_1 + R_0 - lam_0|| / ...
+    Scal mone{nullptr, 0, 0, -1.0};
+    if (!trans) {
+      k_lincomb<<<g, kVT, 0, st>>>(c.Tv, c.vs, one, f->X + 8 * N, 9 * N, mone, f->X, 9 * N, d_ids, N);
       note_launch();
+    } else {
+      k_lincomb<<<g, kVT, 0, st>>>(c.Tv, c.vs, one, f->X, 9 * N, mone, f->X + 8 * N, 9 * N, d_ids, N);
+      note_launch();
+      k_lincomb<<<g, kVT, 0, st>>>(f->X, 9 * N, one, f->X + 8 * N, 9 * N, zero, nullptr, 0, d_ids, N);
+      note_launch();
+      // the sweep leaves lam_tau - R_tau = P_tau^T lam_{tau+1} in bins 1..7
+      for (int t = 1; t < 8; ++t) {
+        k_lincomb<<<g, kVT, 0, st>>>(f->X + t * N, 9 * N, one, f->X + t * N, 9 * N, one, f->E + t * N, 8 * N, d_ids, N);
+        note_launch();
+      }
     }
-  }
-  for (int o = 0; o < n; ++o) mv[o]++;
-  // periodicity: forward ||X8 - X0|| / (||X0|| + 1e-30); adjoint: ||P0^T lam1 + R0 - lam0|| / ...
-  if (!trans) {
-    Scal mone{nullptr, 0, 0, -1.0};
-    k_lincomb<<<g, kVT, 0, st>>>(c.Tv, c.vs, one, f->X + 8 * N, 9 * N, mone, f->X, 9 * N, d_ids, N);
-    note_launch();
-  } else {
-    // lam0_check = P_0^T lam_1 + R_0 computed in place into X[0], then X[0] = lam_0
-    Scal mone{nullptr, 0, 0, -1.0};
-    rc = chain_accurate(c, d_ids, n, f->E, fscale, 0, 1);
-    if (rc) return rc;
-    k_lincomb<<<g, kVT, 0, st>>>(c.Tv, c.vs, one, f->X, 9 * N, mone, c.Xv, c.vs, d_ids, N);
-    note_launch();
-    k_lincomb<<<g, kVT, 0, st>>>(f->X, 9 * N, one, c.Xv, c.vs, zero, nullptr, 0, d_ids, N);
-    note_launch();
-    k_lincomb<<<g, kVT, 0, st>>>(f->X + 8 * N, 9 * N, one, c.Xv, c.vs, zero, nullptr, 0, d_ids, N);
-    note_launch();
-  }
   }
   rc = sqnorm(c, c.Tv, c.vs, d_ids, n, S_TMP);
   if (rc) return rc;
