@@ -676,7 +676,8 @@ int orbit_factor_bytes(orbit_factor_t f, int64_t* numeric_bytes, int64_t* worksp
     *workspace_bytes = (int64_t)2 * f->front_group * S.front_buf_size * vb +
                        (f->tc_pack ? (int64_t)f->front_group * S.tc_pack_size * 4 : 0) +
                        (int64_t)f->n_sets * f->n_bins * 7 * S.N * 8 +
-                       (int64_t)f->n_orbits * (9 + 1 + 8 + 23 + 33) * S.N * 8;
+                       (int64_t)f->n_orbits * (9 + 1 + 8 + 23 + 33) * S.N * 8 + (int64_t)f->flow_bytes +
+                       (f->multi ? (int64_t)2 * f->n_orbits * (S.w_size + 2 * S.N) * vb : 0);
   return ORBIT_OK;
 }
 
