@@ -2439,18 +2439,6 @@ unsigned chain_spin_ns() {
   return v;
 }
 
-// Whether a launch of B groups is bound by its dependency chain rather than by
-// the factor values it reads: up to 40 M factor entries per bin of all groups,
-// 60 M where a group's tree is small (its chunks are few).  k_flow against
-// k_chain, 8 bins, ms: 24x20x15 FP64 1 orbit 0.45 / 0.96, FP32 24 orbits (52 M) 1.54
-// / 1.76; 40x36x15 FP64 4 orbits (37 M) 1.65 / 1.74, FP32 4 1.09 / 1.41; 53x47x13
-// FP64 2 orbits (30 M) 1.32 / 1.40, FP32 4 (59 M) 1.64 / 1.56; 60x54x15 FP64 1 orbit
-// (26 M) 1.27 / 1.35, FP32 2 (53 M) 1.68 / 1.32; 80x72x15 FP64 1 orbit (52 M) 2.4 /
-// 1.7.
-bool chain_bound(const Symbolic& S, int B) {
-  return (int64_t)B * S.fac_nnz <= (S.fac_nnz <= 5000000 ? 60000000 : 40000000);
-}
-
 // The FP32 many-right-hand-side kernels on a prepared launch: groups of K.
 int launch_multi(orbit_factor_s* f, const ChainDev<float>& C, int K, int ks, int B, int trans, double* X,
                  const int* d_orbit_ids, int tau0, const double* E, double escale, int sms, cudaStream_t st) {
@@ -2543,7 +2531,7 @@ int launch_chain_t(orbit_factor_s* f, double* X, int B, const int* d_orbit_ids, 
   const int Bs = multi && sizeof(T) == 4 ? (B + 3) / 4 : Bt;
   const int64_t bin_elems = (int64_t)Bt * S.fac_nnz;
   const int ks = flow && trans ? (bin_elems <= 110000000 && sizeof(T) == 8 ? 0 : bin_elems <= 330000000 ? 1 : 2)
-                               : (Bs <= 2 ? 0 : Bs <= 6 ? 1 : 2);
+                               : (Bs < kSchedGroups[1] ? 0 : Bs < kSchedGroups[2] ? 1 : 2);
   const bool rows = flow && !trans;
   const SolveSched& Q = S.sched[ks];
   const auto& q = sy->d.sched[ks];

@@ -175,6 +175,21 @@ struct SymbolicOptions {
   int periodic_x = 0;     // periodic longitude (needs nx >= 3)
 };
 
+// The fewest groups of a launch that runs each schedule of row chunks.
+constexpr int kSchedGroups[kNumSched] = {1, 3, 7};
+
+// Whether a launch of B groups is bound by its dependency chain rather than by
+// the factor values it reads: up to 40 M factor entries per bin of all groups,
+// 60 M where a group's tree is small (its chunks are few).  k_flow against
+// k_chain, 8 bins, ms: 24x20x15 FP64 1 orbit 0.45 / 0.96, FP32 24 orbits (52 M) 1.54
+// / 1.76; 40x36x15 FP64 4 orbits (37 M) 1.65 / 1.74, FP32 4 1.09 / 1.41; 53x47x13
+// FP64 2 orbits (30 M) 1.32 / 1.40, FP32 4 (59 M) 1.64 / 1.56; 60x54x15 FP64 1 orbit
+// (26 M) 1.27 / 1.35, FP32 2 (53 M) 1.68 / 1.32; 80x72x15 FP64 1 orbit (52 M) 2.4 /
+// 1.7.
+inline bool chain_bound(const Symbolic& S, int64_t B) {
+  return B * S.fac_nnz <= (S.fac_nnz <= 5000000 ? 60000000 : 40000000);
+}
+
 // Build the symbolic analysis.  Returns an empty string on success, an
 // error message otherwise.
 std::string build_symbolic(int nz, int ny, int nx, const SymbolicOptions& opt, Symbolic& S);
