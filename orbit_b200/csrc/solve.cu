@@ -862,15 +862,14 @@ __device__ __noinline__ bool spin_entry(const Entry<T>* p, unsigned tag, int* st
 // when a wait was given up (uniform over the warp).
 template <typename T, int NT, int U, typename Load>
 __device__ __forceinline__ bool flow_gather(int cnt, int* status, long long limit, unsigned max_ns, Load&& load) {
-  for (int base = 0; base < cnt; base += 32 * NT) {
-    const int left = cnt - base - (int)threadIdx.x;
-    const int mine = left > 0 ? min(32, (left + NT - 1) / NT) : 0;
-    const int most = min(32, (cnt - base + NT - 1) / NT);
-    unsigned todo = mine == 32 ? 0xffffffffu : (1u << mine) - 1u;
+  constexpr int kWindow = flow_window(U);
+  for (int base = 0; base < cnt; base += kWindow * NT) {
+    const FlowShare sh = flow_share(cnt, base, (int)threadIdx.x, NT, kWindow);
+    unsigned todo = sh.mine == 32 ? 0xffffffffu : (1u << sh.mine) - 1u;
     for (;;) {
       const Entry<T>* miss = nullptr;
       unsigned miss_tag = 0;
-      for (int j = 0; j < most; j += U) load(base + j * NT + (int)threadIdx.x, j, todo, miss, miss_tag);
+      for (int j = 0; j < sh.most; j += U) load(base + j * NT + (int)threadIdx.x, j, todo, miss, miss_tag);
       const unsigned bad = __ballot_sync(0xffffffffu, todo != 0);
       if (!bad) break;
       bool ok = true;

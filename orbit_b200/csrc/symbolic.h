@@ -52,6 +52,27 @@ int64_t staged_row(int kind, int a, int b, int n, int ldn, int ldm) {
   return kind == 0 ? (last + 3) / 4 * 4 : int64_t(ldn - a / 4 * 4) + ldm;
 }
 
+// Shares of a dataflow gather of cnt positions: rounds of flow_window(U) positions
+// per thread (a multiple of the U it has in flight, so that no U of them reach
+// beyond the 32 bits that mark those still missing), position q by thread q mod
+// nt.  In the round from `base` on, thread tid has `mine` positions and the
+// block's first thread `most`.
+constexpr int flow_window(int U) { return 32 / U * U; }
+struct FlowShare {
+  int mine, most;
+};
+inline
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+FlowShare flow_share(int cnt, int base, int tid, int nt, int window) {
+  const int left = cnt - base - tid, all = (cnt - base + nt - 1) / nt, own = left > 0 ? (left + nt - 1) / nt : 0;
+  FlowShare f;
+  f.mine = own < window ? own : window;
+  f.most = all < window ? all : window;
+  return f;
+}
+
 // One kernel launch of the numeric factorization schedule.
 struct FactorLaunch {
   enum Kind : int { ZERO = 0, SCATTER, EXTEND, DIAG, PANEL, UPDATE, SCHUR, INV, TRIL, PRODL, TRIU, PRODU, TC_PACK, ASSEMBLE, TC_GEMM, FRONT } kind;
