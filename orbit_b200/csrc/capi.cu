@@ -137,19 +137,6 @@ int build_device_symbolic(orbit_symbolic_s* h) {
     ORBIT_TRY(upload(A, &q.nchunk_fwdT, Q.nchunk_fwdT));
     ORBIT_TRY(upload(A, &q.nchunk_bwdT, Q.nchunk_bwdT));
   }
-  for (int k = 0; k < kNumSched && S.max_sub_front == 0; ++k)
-    for (int v = 0; v < 4; ++v) {
-      const FlowSched& Q = v < 2 ? S.staged[k][v] : v == 2 ? S.columns[k] : S.whole[k];
-      DevSym::Flow& q = v < 2 ? d.staged[k][v] : v == 2 ? d.columns[k] : d.whole[k];
-      ORBIT_TRY(upload(A, &q.recs, Q.recs));
-      ORBIT_TRY(upload(A, &q.phase_off, Q.phase_off));
-    }
-  if (S.max_sub_front == 0) {
-    ORBIT_TRY(upload(A, &d.wide.recs, S.wide.recs));
-    ORBIT_TRY(upload(A, &d.wide.phase_off, S.wide.phase_off));
-    ORBIT_TRY(upload(A, &d.wide_nch_f, S.wide_nch_f));
-    ORBIT_TRY(upload(A, &d.wide_nch_b, S.wide_nch_b));
-  }
   ORBIT_TRY(upload(A, &d.perm, S.perm));
   ORBIT_TRY(upload(A, &d.iperm, S.iperm));
   ORBIT_TRY(upload(A, &d.level, S.level));
@@ -176,6 +163,49 @@ constexpr int kDefaultLeaf = 64;
 constexpr int kChunkElems = 8192;
 
 }  // namespace
+
+// One allocation and one copy for a schedule's arrays.
+int flow_table(orbit_symbolic_s* sy, FlowKind kind, int k, cudaStream_t st, const DevSym::Flow** out) {
+  std::lock_guard<std::mutex> lk(sy->mu);
+  DevSym::Flow& q = sy->d.flow[kind][k];
+  *out = &q;
+  if (q.recs) return ORBIT_OK;
+  const FlowSched P = build_flow(sy->S, kind, k);
+  const size_t rb = P.recs.size() * sizeof(FlowRec);
+  const size_t ints = P.phase_off.size() + P.nch_f.size() + P.nch_b.size();
+  std::vector<unsigned char> h(rb + ints * sizeof(int32_t));
+  std::memcpy(h.data(), P.recs.data(), rb);
+  size_t at = rb;
+  for (const std::vector<int32_t>* v : {&P.phase_off, &P.nch_f, &P.nch_b}) {
+    if (!v->empty()) std::memcpy(h.data() + at, v->data(), v->size() * sizeof(int32_t));
+    at += v->size() * sizeof(int32_t);
+  }
+  unsigned char* p = nullptr;
+  ORBIT_TRY(dalloc(sy->allocs, &p, h.size()));
+  ORBIT_CUDA_TRY(cudaMemcpyAsync(p, h.data(), h.size(), cudaMemcpyHostToDevice, st));
+  ORBIT_CUDA_TRY(cudaStreamSynchronize(st));  // other handles' streams may read it next
+  q.phase_off = reinterpret_cast<int32_t*>(p + rb);
+  q.nch_f = q.phase_off + P.phase_off.size();
+  q.nch_b = q.nch_f + P.nch_f.size();
+  q.items_per_bin = P.items_per_bin;
+  q.recs = reinterpret_cast<FlowRec*>(p);
+  return ORBIT_OK;
+}
+
+int sweep_buffers(orbit_factor_s* f, bool multi) {
+  const Symbolic& S = f->sym->S;
+  const size_t bytes = 2 * (size_t)f->n_orbits * (S.w_size + 2 * S.N) * (f->precision == ORBIT_PREC_FP32 ? 4 : 8);
+  if (multi && !f->multi) {
+    // whole groups of 16, 8 or 4: fewer than twice the orbits
+    ORBIT_TRY(dalloc(f->allocs, reinterpret_cast<unsigned char**>(&f->multi), bytes));
+    f->multi_bytes = bytes;
+  } else if (!multi && !f->flow) {
+    ORBIT_TRY(dalloc(f->allocs, &f->flow, bytes));  // value and tag
+    f->flow_bytes = bytes;
+  }
+  return ORBIT_OK;
+}
+
 }  // namespace orbit
 
 using namespace orbit;
@@ -549,15 +579,6 @@ int orbit_factor_create_ex(orbit_symbolic_t sym, int n_orbits, int n_sets, int n
   if ((rc = dalloc(A, &f->Ybuf, (size_t)n_orbits * N))) return fail(rc);
   if ((rc = dalloc(A, &f->Wbuf, (size_t)n_orbits * S.w_size))) return fail(rc);
   if ((rc = dalloc(A, &f->counters, (size_t)n_orbits * 16 * S.nsuper))) return fail(rc);
-  if (S.max_sub_front == 0) {
-    f->flow_bytes = 2 * vb * (size_t)n_orbits * (S.w_size + 2 * N);
-    if ((rc = dalloc(A, &f->flow, f->flow_bytes))) return fail(rc);
-    if (cudaMemset(f->flow, 0, f->flow_bytes) != cudaSuccess) return fail(ORBIT_ERR_CUDA);
-    if (precision == ORBIT_PREC_FP32 && n_sets == 1 && n_orbits > 1) {
-      // whole groups of 16, 8 or 4: fewer than twice the orbits
-      if ((rc = dalloc(A, &f->multi, (size_t)2 * n_orbits * (S.w_size + 2 * N)))) return fail(rc);
-    }
-  }
   if ((rc = dalloc(A, &f->E, (size_t)n_orbits * 8 * N))) return fail(rc);
   if ((rc = dalloc(A, &f->tmpv, (size_t)n_orbits * 23 * N))) return fail(rc);
   if ((rc = dalloc(A, &f->orbit_ids, (size_t)n_orbits))) return fail(rc);
@@ -583,6 +604,9 @@ int orbit_factor_create_ex(orbit_symbolic_t sym, int n_orbits, int n_sets, int n
     return fail(ORBIT_ERR_NOMEM);
   }
   if (cudaMemset(f->status, 0, sizeof(int)) != cudaSuccess) return fail(ORBIT_ERR_CUDA);
+  // what the forward sweeps of all slots take; the other sweeps' is made when
+  // they first run
+  if ((rc = prepare_sweeps(f, n_orbits, 0, nullptr))) return fail(rc);
   *out = f;
   return ORBIT_OK;
 }
@@ -677,7 +701,7 @@ int orbit_factor_bytes(orbit_factor_t f, int64_t* numeric_bytes, int64_t* worksp
                        (f->tc_pack ? (int64_t)f->front_group * S.tc_pack_size * 4 : 0) +
                        (int64_t)f->n_sets * f->n_bins * 7 * S.N * 8 +
                        (int64_t)f->n_orbits * (9 + 1 + 8 + 23 + 33) * S.N * 8 + (int64_t)f->flow_bytes +
-                       (f->multi ? (int64_t)2 * f->n_orbits * (S.w_size + 2 * S.N) * vb : 0);
+                       (int64_t)f->multi_bytes;
   return ORBIT_OK;
 }
 

@@ -24,11 +24,12 @@ struct DevSym {
     int32_t *phase_off = nullptr, *phase_offT = nullptr;
     int32_t *nchunk_fwd = nullptr, *nchunk_bwd = nullptr, *nchunk_fwdT = nullptr, *nchunk_bwdT = nullptr;
   } sched[orbit::kNumSched];
+  // dataflow schedules, each made and uploaded when a launch first takes it
   struct Flow {
     orbit::FlowRec *recs = nullptr;
-    int32_t *phase_off = nullptr;
-  } staged[orbit::kNumSched][2], columns[orbit::kNumSched], whole[orbit::kNumSched], wide;
-  int32_t *wide_nch_f = nullptr, *wide_nch_b = nullptr;
+    int32_t *phase_off = nullptr, *nch_f = nullptr, *nch_b = nullptr;
+    int32_t items_per_bin = 0;
+  } flow[orbit::kFlowKinds][orbit::kNumSched];
   int32_t *perm = nullptr, *iperm = nullptr;
   int32_t *level = nullptr;
   int64_t *tc_pack_off = nullptr;
@@ -75,12 +76,14 @@ struct orbit_factor_s {
   double* Wbuf = nullptr;   // w_size
   int* counters = nullptr;  // 8 * 2 * nsuper
   // tagged results of the dataflow chain kernels, all orbits: w_size update
-  // entries, N forward results and N solutions each
+  // entries, N forward results and N solutions each; made when a launch first
+  // takes those kernels
   unsigned char* flow = nullptr;
   size_t flow_bytes = 0;
-  // interleaved results of the FP32 many-right-hand-side kernels
+  // interleaved results of the FP32 many-right-hand-side kernels, likewise
   float* multi = nullptr;
-  unsigned flow_seq = 0;    // launches so far (28 bits), the tags' high part
+  size_t multi_bytes = 0;
+  unsigned flow_seq = 0x0fffffffu;  // launches (28 bits), the tags' high part; the first starts over
   double* E = nullptr;      // 8 N forcing (new order)
   double* tmpv = nullptr;   // 4 N scratch vectors
   int* orbit_ids = nullptr; // n_orbits
@@ -105,3 +108,12 @@ struct orbit_factor_s {
   std::mutex mu;
   std::vector<void*> allocs;
 };
+
+namespace orbit {
+// Device table of one dataflow schedule (the arguments of build_flow).
+int flow_table(orbit_symbolic_s* sy, FlowKind kind, int k, cudaStream_t st, const DevSym::Flow** out);
+// The handle's tagged (multi: interleaved) buffers.
+int sweep_buffers(orbit_factor_s* f, bool multi);
+// What the sweeps of B slots need beside the handle's own: both of the above.
+int prepare_sweeps(orbit_factor_s* f, int B, int trans, cudaStream_t st);
+}  // namespace orbit

@@ -2439,8 +2439,9 @@ unsigned chain_spin_ns() {
 }
 
 // The FP32 many-right-hand-side kernels on a prepared launch: groups of K.
-int launch_multi(orbit_factor_s* f, const ChainDev<float>& C, int K, int ks, int B, int trans, double* X,
-                 const int* d_orbit_ids, int tau0, const double* E, double escale, int sms, cudaStream_t st) {
+int launch_multi(orbit_factor_s* f, const ChainDev<float>& C, int K, const DevSym::Flow& p, int B, int trans,
+                 double* X, const int* d_orbit_ids, int tau0, const double* E, double escale, int sms,
+                 cudaStream_t st) {
   const Symbolic& S = f->sym->S;
   MultiDev M;
   M.C = C;
@@ -2448,18 +2449,12 @@ int launch_multi(orbit_factor_s* f, const ChainDev<float>& C, int K, int ks, int
   M.W = f->multi;
   M.Y = M.W + groups * S.w_size * K;
   M.X = M.Y + groups * S.N * K;
-  M.nch_f = C.nch_f;
-  M.nch_b = C.nch_b;
-  const FlowSched& P = trans ? S.wide : S.whole[ks];
-  const DevSym::Flow& p = trans ? f->sym->d.wide : f->sym->d.whole[ks];
+  M.nch_f = trans ? p.nch_f : C.nch_f;
+  M.nch_b = trans ? p.nch_b : C.nch_b;
   M.C.recs = p.recs;
   M.C.phase_off = p.phase_off;
-  M.C.items_per_bin = P.items_per_bin;
-  M.C.total = (C.tau1 - C.tau0) * P.items_per_bin * C.B;
-  if (trans) {
-    M.nch_f = f->sym->d.wide_nch_f;
-    M.nch_b = f->sym->d.wide_nch_b;
-  }
+  M.C.items_per_bin = p.items_per_bin;
+  M.C.total = (C.tau1 - C.tau0) * p.items_per_bin * C.B;
   const void* fn = K == 16 ? (trans ? (const void*)k_multi<16, true> : (const void*)k_multi<16, false>)
                    : K == 8 ? (trans ? (const void*)k_multi<8, true> : (const void*)k_multi<8, false>)
                             : (trans ? (const void*)k_multi<4, true> : (const void*)k_multi<4, false>);
@@ -2498,6 +2493,58 @@ int launch_multi(orbit_factor_s* f, const ChainDev<float>& C, int K, int ks, int
   return ORBIT_OK;
 }
 
+// Which kernel, chunk schedule and dataflow table (kFlowKinds: none) a launch of
+// B slots takes.
+struct SweepRoute {
+  bool multi, flow, rows;  // many right-hand sides per task; tagged values; of row chunks
+  int K, groups;           // right-hand sides per task, task groups per (node chunk, bin)
+  int ks;
+  FlowKind kind;
+  int k;
+};
+
+SweepRoute sweep_route(const orbit_factor_s* f, int B, int trans, bool never_ready) {
+  const Symbolic& S = f->sym->S;
+  const bool fp32 = f->precision == ORBIT_PREC_FP32, sub = S.max_sub_front > 0;
+  SweepRoute r;
+  // Right-hand sides on one factor set go through the multi-RHS kernels in
+  // groups of K (row-chunk tasks, forward and transposed sweeps).
+  r.multi = !never_ready && f->n_sets == 1 && B >= 2 && !sub;
+  // group size: FP64 2, FP32 the batch's, while its vectors leave a block resident
+  r.K = !r.multi ? 1 : !fp32 ? 2 : B > 8 ? 16 : B > 4 ? 8 : 4;
+  while (r.K > 4 && (size_t)(S.max_front + 16) * r.K * sizeof(float) > 215000) r.K /= 2;
+  r.groups = (B + r.K - 1) / r.K;
+  // dataflow kernels: the transposed sweeps, and the others of launches bound
+  // by their dependency chain
+  r.flow = !r.multi && !sub && (trans || never_ready || chain_bound(S, r.groups));
+  r.rows = r.flow && !trans;
+  // Schedule by batch size: small chunks shorten one orbit's critical path,
+  // large ones cut per-task overhead when many orbits fill the GPU.  The
+  // transposed dataflow sweeps, whose sums do not depend on the chunks, go by
+  // the factor entries that one bin's sweep of all groups reads instead (2 and
+  // 6 groups of the 80x72x15 grid's 52 M).
+  // (The FP32 many-right-hand-side rows keep the schedule of groups of four,
+  // from which their lanes per row, and so the order of their sums, follow.)
+  const int Bs = r.multi && fp32 ? (B + 3) / 4 : r.groups;
+  const int64_t bin_elems = (int64_t)Bs * S.fac_nnz;
+  r.ks = r.flow && trans ? (bin_elems <= 110000000 && !fp32 ? 0 : bin_elems <= 330000000 ? 1 : 2)
+                         : (Bs < kSchedGroups[1] ? 0 : Bs < kSchedGroups[2] ? 1 : 2);
+  const bool wide = r.multi && trans;
+  r.kind = r.multi ? (!fp32 ? kFlowKinds : wide ? kFlowWide : kFlowWhole)
+           : !r.flow ? kFlowKinds : trans ? kFlowColumns : fp32 ? kFlowRows32 : kFlowRows64;
+  r.k = wide ? 0 : r.ks;
+  return r;
+}
+
+// The launch's dataflow table (null where it takes none) and the handle's
+// buffers for it.
+int sweep_resources(orbit_factor_s* f, const SweepRoute& r, cudaStream_t st, const DevSym::Flow** table) {
+  *table = nullptr;
+  if (r.kind == kFlowKinds) return ORBIT_OK;
+  if (int rc = sweep_buffers(f, r.multi)) return rc;
+  return flow_table(f->sym, r.kind, r.k, st, table);
+}
+
 template <typename T>
 int launch_chain_t(orbit_factor_s* f, double* X, int B, const int* d_orbit_ids, int trans, int tau0,
                    int tau1, const double* E, double escale, cudaStream_t st, bool never_ready = false) {
@@ -2507,31 +2554,12 @@ int launch_chain_t(orbit_factor_s* f, double* X, int B, const int* d_orbit_ids, 
   D.first = sy->d.first; D.n = sy->d.n; D.m = sy->d.m; D.parent = sy->d.parent;
   D.child = sy->d.child; D.uidx = sy->d.uidx; D.rel = sy->d.rel; D.ldn = sy->d.ldn; D.ldm = sy->d.ldm;
   D.ginv = sy->d.ginv; D.ginv_off = sy->d.ginv_off;
-  // Right-hand sides on one factor set go through the multi-RHS kernels in
-  // groups of K (row-chunk tasks, forward and transposed sweeps).
-  const bool multi = !never_ready && f->n_sets == 1 && B >= 2 && S.max_sub_front == 0;
+  const SweepRoute r = sweep_route(f, B, trans, never_ready);
+  const DevSym::Flow* table = nullptr;
+  if (int rc = sweep_resources(f, r, st, &table)) return rc;
+  const bool multi = r.multi, flow = r.flow, rows = r.rows, sub = S.max_sub_front > 0;
+  const int Bt = r.groups, ks = r.ks;
   constexpr int KM = 2;  // FP64 group size
-  // FP32 group size: the batch's, while its vectors leave a block resident
-  int KF = B > 8 ? 16 : B > 4 ? 8 : 4;
-  while (KF > 4 && (size_t)(S.max_front + 16) * KF * sizeof(float) > 215000) KF /= 2;
-  const int Kg = !multi ? 1 : sizeof(T) == 4 ? KF : KM;
-  const int Bt = (B + Kg - 1) / Kg;  // task groups per (node chunk, bin)
-  // dataflow kernels: the transposed sweeps, and the others of launches bound
-  // by their dependency chain
-  const bool sub = S.max_sub_front > 0;
-  const bool flow = !multi && !sub && (trans || never_ready || chain_bound(S, Bt));
-  // Schedule by batch size: small chunks shorten one orbit's critical path,
-  // large ones cut per-task overhead when many orbits fill the GPU.  The
-  // transposed dataflow sweeps, whose sums do not depend on the chunks, go by
-  // the factor entries that one bin's sweep of all groups reads instead (2 and
-  // 6 groups of the 80x72x15 grid's 52 M).
-  // (The FP32 many-right-hand-side rows keep the schedule of groups of four,
-  // from which their lanes per row, and so the order of their sums, follow.)
-  const int Bs = multi && sizeof(T) == 4 ? (B + 3) / 4 : Bt;
-  const int64_t bin_elems = (int64_t)Bt * S.fac_nnz;
-  const int ks = flow && trans ? (bin_elems <= 110000000 && sizeof(T) == 8 ? 0 : bin_elems <= 330000000 ? 1 : 2)
-                               : (Bs < kSchedGroups[1] ? 0 : Bs < kSchedGroups[2] ? 1 : 2);
-  const bool rows = flow && !trans;
   const SolveSched& Q = S.sched[ks];
   const auto& q = sy->d.sched[ks];
   D.nch_f = trans ? q.nchunk_fwdT : q.nchunk_fwd;
@@ -2543,11 +2571,9 @@ int launch_chain_t(orbit_factor_s* f, double* X, int B, const int* d_orbit_ids, 
   D.phase_off = trans ? q.phase_offT : q.phase_off;
   D.items_per_bin = trans ? Q.items_per_binT : Q.items_per_bin;
   if (flow) {
-    const FlowSched& P = rows ? S.staged[ks][sizeof(T) == 8] : S.columns[ks];
-    const DevSym::Flow& p = rows ? sy->d.staged[ks][sizeof(T) == 8] : sy->d.columns[ks];
-    D.recs = p.recs;
-    D.phase_off = p.phase_off;
-    D.items_per_bin = P.items_per_bin;
+    D.recs = table->recs;
+    D.phase_off = table->phase_off;
+    D.items_per_bin = table->items_per_bin;
   }
   D.nphase = 2 * S.nlevels;
   if (D.nphase > kMaxPhases) {
@@ -2584,12 +2610,14 @@ int launch_chain_t(orbit_factor_s* f, double* X, int B, const int* d_orbit_ids, 
   if (D.total <= 0) return ORBIT_OK;
   if (flow) {
     // tags of this launch: 16 per launch, never 0 or all ones; a handle's
-    // buffers are cleared each time its 28-bit launch count starts over
-    f->flow_seq = (f->flow_seq + 1) & 0x0fffffffu;
-    if (f->flow_seq == 0) {
+    // buffers are cleared, on this stream, each time its 28-bit launch count
+    // starts over, the first launch being one of those
+    unsigned seq = (f->flow_seq + 1) & 0x0fffffffu;
+    if (seq == 0) {
       ORBIT_CUDA_TRY(cudaMemsetAsync(f->flow, 0, f->flow_bytes, st));
-      f->flow_seq = 1;
+      seq = 1;
     }
+    f->flow_seq = seq;
     D.tag0 = f->flow_seq * 16u + 1u;
     const size_t eb = sizeof(Entry<T>);
     unsigned char* p = f->flow;
@@ -2604,7 +2632,7 @@ int launch_chain_t(orbit_factor_s* f, double* X, int B, const int* d_orbit_ids, 
       rows ? kStageBytes + sizeof(T) * ((size_t)S.max_front + 8)
            : sizeof(T) * ((size_t)kWarps * 32 * (flow && sizeof(T) == 4 ? 4 : 1) +
                           std::max<size_t>(S.max_front + 8, (size_t)kWarps * ((S.max_sub_front + 7) & ~3)) + 8);
-  const bool few = (double)bin_elems * sizeof(T) <= kChainManyBytes[sizeof(T) == 8];
+  const bool few = (double)Bt * S.fac_nnz * sizeof(T) <= kChainManyBytes[sizeof(T) == 8];
   const void* kfn = rows    ? (const void*)k_flow<T>
                     : flow  ? (const void*)k_flow_t<T>
                     : !sub  ? (few ? (const void*)k_chain<T, false, false, true> : (const void*)k_chain<T, false, false, false>)
@@ -2618,7 +2646,7 @@ int launch_chain_t(orbit_factor_s* f, double* X, int B, const int* d_orbit_ids, 
   ORBIT_CUDA_TRY(cudaGetDevice(&dev));
   ORBIT_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   if constexpr (sizeof(T) == 4)
-    if (multi) return launch_multi(f, D, KF, ks, B, trans, X, d_orbit_ids, tau0, E, escale, sms, st);
+    if (multi) return launch_multi(f, D, r.K, *table, B, trans, X, d_orbit_ids, tau0, E, escale, sms, st);
   if constexpr (sizeof(T) == 8) if (multi) {
     const int vcap = (S.max_front + 8 + 3) & ~3;
     const size_t msmem = sizeof(T) * ((size_t)KM * vcap + (size_t)KM * kWarps * 32);
@@ -2691,6 +2719,11 @@ int launch_chain_t(orbit_factor_s* f, double* X, int B, const int* d_orbit_ids, 
 }
 
 }  // namespace
+
+int prepare_sweeps(orbit_factor_s* f, int B, int trans, cudaStream_t st) {
+  const DevSym::Flow* table = nullptr;
+  return sweep_resources(f, sweep_route(f, B, trans, false), st, &table);
+}
 
 // Run the chain on f->X (per orbit 9 vectors in permuted order).  Forward:
 // reads X[tau0], writes X[tau0+1..tau1].  Transposed: reads X[tau1], writes

@@ -632,115 +632,104 @@ std::string build_symbolic(int nz, int ny, int nx, const SymbolicOptions& opt, S
     Q.phase_offT.push_back(int32_t(Q.sitems.size() / 4) - base);
     Q.items_per_binT = Q.phase_offT.back();
   }
-  auto flow_rec = [&](int s, int r0, int r1, int kind, int len) {
+  return std::string();
+}
+
+FlowSched build_flow(const Symbolic& S, FlowKind kind, int k) {
+  FlowSched P;
+  const int ns = S.nsuper;
+  auto flow_rec = [&](int s, int r0, int r1, int task, int len) {
     FlowRec r;
-    r.s = s; r.r0 = r0; r.r1 = r1; r.kind_len = kind + 256 * len;
+    r.s = s; r.r0 = r0; r.r1 = r1; r.kind_len = task + 256 * len;
     r.n = S.n[s]; r.m = S.m[s]; r.first = S.first[s]; r.ldn = S.ldn[s]; r.ldm = S.ldm[s];
     r.woff = int32_t(S.woff[s]);
     const int c0 = S.child[2 * s], c1 = S.child[2 * s + 1];
     r.w0 = c0 >= 0 ? int32_t(S.woff[c0]) : -1;
     r.w1 = c1 >= 0 ? int32_t(S.woff[c1]) : -1;
     r.fac_off = S.fac_off[s];
-    r.map_off = (kind & 1) == 0 ? S.ginv_off[s] : S.uoff[s];
+    r.map_off = (task & 1) == 0 ? S.ginv_off[s] : S.uoff[s];
     return r;
   };
-  // Column chunks of the transposed dataflow sweeps: vectors of consecutive
-  // columns, so a chunk starts at a multiple of 32 columns of its block (SQ
-  // below column n, Qr from n on; of 16 in the small-batch schedule, whose chunks
-  // at the tree's top would be too few otherwise) and does not straddle the two.
-  for (int k = 0; k < kNumSched && S.max_sub_front == 0; ++k) {
-    FlowSched& P = S.columns[k];
+  if (kind == kFlowColumns || kind == kFlowWide) {
+    // Column chunks.  Those of the transposed dataflow sweeps are vectors of
+    // consecutive columns, so a chunk starts at a multiple of 32 columns of its
+    // block (SQ below column n, Qr from n on; of 16 in the small-batch schedule,
+    // whose chunks at the tree's top would be too few otherwise) and does not
+    // straddle the two.
     const int64_t elems = S.sched[k].chunk_elems;
     const int grain = k == 0 ? 16 : 32;
-    auto chunks = [&](int s, int kind) {
-      const int n = S.n[s], m = S.m[s], cols = kind == 2 ? n + m : n;
+    auto columns = [&](int s, int task) {
+      const int n = S.n[s], m = S.m[s], cols = task == 2 ? n + m : n;
       int64_t acc = 0;
       for (int c = 0, start = 0; c < cols; ++c) {
-        acc += (kind == 2 ? std::min(c + 1, n) : n - c + m) + 8;
+        acc += (task == 2 ? std::min(c + 1, n) : n - c + m) + 8;
         const int at = c + 1 - (c >= n ? n : 0);
         if ((acc >= elems && at % grain == 0) || c == n - 1 || c == cols - 1) {
-          P.recs.push_back(flow_rec(s, start, c + 1, kind, 0));
+          P.recs.push_back(flow_rec(s, start, c + 1, task, 0));
           start = c + 1;
           acc = 0;
         }
       }
     };
-    for (int l = S.nlevels - 1; l >= 0; --l) {
-      P.phase_off.push_back(int32_t(P.recs.size()));
-      for (int s : S.level_sups[l]) chunks(s, 2);
-    }
-    for (int l = 0; l < S.nlevels; ++l) {
-      P.phase_off.push_back(int32_t(P.recs.size()));
-      for (int s : S.level_sups[l]) chunks(s, 3);
-    }
-    P.phase_off.push_back(int32_t(P.recs.size()));
-    P.items_per_bin = P.phase_off.back();
-  }
-  if (S.max_sub_front == 0) {
-    FlowSched& P = S.wide;
-    S.wide_nch_f.assign(ns, 0);
-    S.wide_nch_b.assign(ns, 0);
-    auto chunks = [&](int s, int kind) {
+    auto wide = [&](int s, int task) {
       // cut at column n: 64 columns where they are long, else as many blocks of
       // 128 as make a task of 32 K entries (forward tasks gather once for all)
-      const int n = S.n[s], cols = kind == 2 ? n + S.m[s] : n;
+      const int n = S.n[s], cols = task == 2 ? n + S.m[s] : n;
       for (int c = 0; c < cols;) {
-        const int rows = kind == 2 ? n : n - c + S.m[s];
-        const int width = rows > 400 ? 64 : kind == 2 ? 128 * std::max(1, 256 / rows) : 128;
+        const int rows = task == 2 ? n : n - c + S.m[s];
+        const int width = rows > 400 ? 64 : task == 2 ? 128 * std::max(1, 256 / rows) : 128;
         const int e = std::min(c + width, c < n ? n : cols);
-        P.recs.push_back(flow_rec(s, c, e, kind, 0));
-        ++(kind == 2 ? S.wide_nch_f : S.wide_nch_b)[s];
+        P.recs.push_back(flow_rec(s, c, e, task, 0));
+        ++(task == 2 ? P.nch_f : P.nch_b)[s];
         c = e;
       }
     };
-    for (int l = S.nlevels - 1; l >= 0; --l) {
-      P.phase_off.push_back(int32_t(P.recs.size()));
-      for (int s : S.level_sups[l]) chunks(s, 2);
+    if (kind == kFlowWide) {
+      P.nch_f.assign(ns, 0);
+      P.nch_b.assign(ns, 0);
     }
-    for (int l = 0; l < S.nlevels; ++l) {
+    auto phase = [&](int l, int task) {
       P.phase_off.push_back(int32_t(P.recs.size()));
-      for (int s : S.level_sups[l]) chunks(s, 3);
-    }
-    P.phase_off.push_back(int32_t(P.recs.size()));
-    P.items_per_bin = P.phase_off.back();
-  }
-  for (int k = 0; k < kNumSched && S.max_sub_front == 0; ++k)
-    for (int prec = 0; prec < 3; ++prec) {  // FP32, FP64, uncut
-      const SolveSched& Q = S.sched[k];
-      FlowSched& P = prec < 2 ? S.staged[k][prec] : S.whole[k];
-      // staged rows only where some launch takes them; the first schedule's
-      // always, for the bounded wait's self-test (80x72x15: the analysis takes 104 ms
-      // with all of them, 79 with these, 74 without any dataflow schedule)
-      if (prec < 2 && k > 0 && !chain_bound(S, kSchedGroups[k])) continue;
-      P.recs.reserve(size_t(Q.items_per_bin) * (prec == 0 ? 2 : prec == 1 ? 4 : 1));
-      const int64_t vb = prec ? 8 : 4;
-      size_t ph = 0;
-      for (int32_t i = 0; i < Q.items_per_bin; ++i) {
-        while (ph < Q.phase_off.size() && Q.phase_off[ph] == i) {
-          P.phase_off.push_back(int32_t(P.recs.size()));
-          ++ph;
-        }
-        const int32_t* it = Q.sitems.data() + 4 * size_t(i);
-        const int s = it[0], kind = it[3], n = S.n[s], m = S.m[s];
-        const int len = kind == 0 ? std::min(it[2] - 1, n) : n - it[1] + m;
-        for (int a = it[1]; a < it[2];) {
-          int b = prec < 2 ? a + 1 : it[2];
-          while (b < it[2]) {
-            const int64_t full = (b + 1 - a) * staged_row(kind, a, b + 1, n, S.ldn[s], S.ldm[s]) * vb;
-            if (full > kStageBytes || (full > kStageBytesCut && b - a >= 4)) break;
-            ++b;
-          }
-          P.recs.push_back(flow_rec(s, a, b, kind, len));
-          a = b;
-        }
+      for (int s : S.level_sups[l]) {
+        if (kind == kFlowWide) wide(s, task);
+        else columns(s, task);
       }
-      while (ph < Q.phase_off.size()) {
+    };
+    for (int l = S.nlevels - 1; l >= 0; --l) phase(l, 2);
+    for (int l = 0; l < S.nlevels; ++l) phase(l, 3);
+    P.phase_off.push_back(int32_t(P.recs.size()));
+  } else {
+    const SolveSched& Q = S.sched[k];
+    const bool whole = kind == kFlowWhole;
+    const int64_t vb = kind == kFlowRows32 ? 4 : 8;
+    P.recs.reserve(size_t(Q.items_per_bin) * (whole ? 1 : kind == kFlowRows32 ? 2 : 4));
+    size_t ph = 0;
+    for (int32_t i = 0; i < Q.items_per_bin; ++i) {
+      while (ph < Q.phase_off.size() && Q.phase_off[ph] == i) {
         P.phase_off.push_back(int32_t(P.recs.size()));
         ++ph;
       }
-      P.items_per_bin = P.phase_off.back();
+      const int32_t* it = Q.sitems.data() + 4 * size_t(i);
+      const int s = it[0], task = it[3], n = S.n[s], m = S.m[s];
+      const int len = task == 0 ? std::min(it[2] - 1, n) : n - it[1] + m;
+      for (int a = it[1]; a < it[2];) {
+        int b = whole ? it[2] : a + 1;
+        while (b < it[2]) {
+          const int64_t full = (b + 1 - a) * staged_row(task, a, b + 1, n, S.ldn[s], S.ldm[s]) * vb;
+          if (full > kStageBytes || (full > kStageBytesCut && b - a >= 4)) break;
+          ++b;
+        }
+        P.recs.push_back(flow_rec(s, a, b, task, len));
+        a = b;
+      }
     }
-  return std::string();
+    while (ph < Q.phase_off.size()) {
+      P.phase_off.push_back(int32_t(P.recs.size()));
+      ++ph;
+    }
+  }
+  P.items_per_bin = P.phase_off.back();
+  return P;
 }
 
 }  // namespace orbit

@@ -115,8 +115,16 @@ static_assert(sizeof(FlowRec) == 64, "loaded as four 16-byte vectors");
 struct FlowSched {
   std::vector<FlowRec> recs;
   std::vector<int32_t> phase_off;
+  std::vector<int32_t> nch_f, nch_b;  // kFlowWide: each supernode's number of chunks
   int32_t items_per_bin = 0;
 };
+// Schedules of the dataflow kernels, by what they are made from: the
+// non-transposed chunks of one of the analysis' schedules cut into staged tasks
+// for FP32 or FP64 factors (a row keeps the lanes of its uncut chunk, and with
+// them the order of its sum) or uncut, their transposed counterparts (column
+// chunks, both precisions), and the column chunks of the many-right-hand-side
+// transposed sweeps.
+enum FlowKind : int { kFlowRows32 = 0, kFlowRows64, kFlowWhole, kFlowColumns, kFlowWide, kFlowKinds };
 
 struct Symbolic {
   int nz = 0, ny = 0, nx = 0;
@@ -158,17 +166,6 @@ struct Symbolic {
   std::vector<int32_t> fitems;            // 4 ints per item
   std::vector<FactorLaunch> fsched;
   SolveSched sched[kNumSched];  // chunk/2, chunk, 2 chunk; sched[1] is the default
-  // the non-transposed chunks of sched[k] cut into staged tasks, for FP32 (0)
-  // and FP64 (1) factors.  A row keeps the lanes of its uncut chunk, and with
-  // them the order of its sum.
-  FlowSched staged[kNumSched][2];
-  FlowSched whole[kNumSched];  // and uncut
-  // their transposed counterparts (column chunks, both precisions)
-  FlowSched columns[kNumSched];
-  // column chunks of the many-right-hand-side transposed sweeps, and each
-  // supernode's number of them
-  FlowSched wide;
-  std::vector<int32_t> wide_nch_f, wide_nch_b;
   std::vector<int32_t> role;  // 0 chunked node, 1 subtree-task root, 2 inside a subtree
   int max_front = 0;
   int max_sub_front = 0;  // largest n+m of a supernode inside a subtree task
@@ -214,5 +211,11 @@ inline bool chain_bound(const Symbolic& S, int64_t B) {
 // Build the symbolic analysis.  Returns an empty string on success, an
 // error message otherwise.
 std::string build_symbolic(int nz, int ny, int nx, const SymbolicOptions& opt, Symbolic& S);
+
+// The dataflow schedule of one kind, from the analysis' schedule k (kFlowWide: 0).
+// Only for analyses without whole-subtree tasks.  Made when a launch first takes
+// it: all of them at once made the analysis 10 to 20 % longer (80x72x15 50 -> 57
+// ms) and their upload 2 to 5 ms of an analysis' first handle.
+FlowSched build_flow(const Symbolic& S, FlowKind kind, int k);
 
 }  // namespace orbit

@@ -1,0 +1,107 @@
+"""What the dataflow sweeps keep beside a factor handle (B200).
+
+A handle is made with what the forward sweeps of all its slots take; the
+schedules and buffers of other sweeps are made, cleared on the launch's stream
+and counted when a launch first takes them.
+"""
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(shape, sets, seed=5):
+    import torch
+    from orbit_b200 import device, synthetic
+    met = synthetic.make_met(seed, *shape, cmfmc_frac=0.3)
+    T = [device.assemble_transport(device.MetDevice(g)) for g in met]
+    d = [torch.as_tensor(v, device="cuda") for q in range(sets)
+         for v in synthetic.make_species(seed + 1 + q, *shape).sink_diag(met)]
+    return [t for _ in range(sets) for t in T], d
+
+
+def _tagged(sym, slots, bits):
+    """Bytes of the tagged, or of the interleaved, results of all slots."""
+    return 2 * slots * (sym.info["update_len"] + 2 * sym.N) * bits // 8
+
+
+def test_made_by_the_launches_that_take_them():
+    import torch
+    from orbit_b200 import device
+    from orbit_b200.symbolic import Symbolic
+    shape = (6, 10, 12)
+    sym = Symbolic(*shape)
+    T, d = _inputs(shape, 1)
+    fb = device.FactorBatch(sym, 5, 32, n_sets=1)
+    fb.numeric(T, d)
+    made = fb.bytes()[1]
+    x = torch.exp(torch.randn(5, sym.N, dtype=torch.float64, device="cuda"))
+    torch.cuda.synchronize()
+    st = torch.cuda.Stream()
+    with torch.cuda.stream(st):
+        fb.chain(x, refine=False)
+        fb.chain(x, trans=True, refine=False)
+        assert fb.bytes()[1] == made  # five slots of one set: the interleaved ones, from the start
+        one = fb.chain(x[:1], trans=True, refine=False)
+        assert fb.bytes()[1] == made + _tagged(sym, 5, 32)
+        assert torch.equal(fb.chain(x[:1], trans=True, refine=False), one)
+    own = device.FactorBatch(sym, 1, 32)
+    own.numeric(T, d)
+    assert torch.equal(own.chain(x[:1], trans=True, refine=False), one)
+
+
+def test_large_batches_hold_none_until_transposed():
+    import torch
+    from orbit_b200 import device
+    from orbit_b200.symbolic import Symbolic
+    shape = (15, 54, 60)
+    sym = Symbolic(*shape)
+    assert 2 * sym.lunz > 40e6  # two slots' forward sweep is not bound by its chain
+    fixed = device.FactorBatch(sym, 1, 32, n_sets=2)  # one slot's is
+    two = device.FactorBatch(sym, 2, 32)
+    per_slot = 8 * 74 * sym.N
+    assert two.bytes()[1] + _tagged(sym, 1, 32) == fixed.bytes()[1] + per_slot
+    T, d = _inputs(shape, 2)
+    two.numeric(T, d)
+    x = torch.exp(torch.randn(2, sym.N, dtype=torch.float64, device="cuda"))
+    before = two.bytes()[1]
+    two.chain(x, refine=False)
+    assert two.bytes()[1] == before
+    two.chain(x, trans=True, refine=False)
+    assert two.bytes()[1] == before + _tagged(sym, 2, 32)
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+def test_first_sweeps_of_two_handles_at_once(bits):
+    import torch
+    from orbit_b200 import device
+    from orbit_b200.symbolic import Symbolic
+    shape = (9, 23, 29)
+    T, d = _inputs(shape, 1)
+    x = torch.exp(torch.randn(1, int(np.prod(shape)), dtype=torch.float64, device="cuda"))
+    sym = Symbolic(*shape)  # its transposed schedule is not there yet
+    handles = [device.FactorBatch(sym, 1, bits) for _ in range(2)]
+    for fb in handles:
+        fb.numeric(T, d)
+    torch.cuda.synchronize()
+    out, gate = [None, None], threading.Barrier(2)
+
+    def sweep(q):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            gate.wait()
+            out[q] = [handles[q].chain(x, trans=t, refine=False) for t in (True, False)]
+            torch.cuda.current_stream().synchronize()
+
+    threads = [threading.Thread(target=sweep, args=(q,)) for q in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for a, b in zip(*out):
+        assert torch.equal(a, b)
+    ref = device.FactorBatch(Symbolic(*shape), 1, bits)
+    ref.numeric(T, d)
+    for a, trans in zip(out[0], (True, False)):
+        assert torch.equal(ref.chain(x, trans=trans, refine=False), a)
