@@ -81,9 +81,13 @@ class _Entry:
         vb = 4 if precision == 32 else 8
         info = sym.info
         scratch = 2 * info["front_elems"] * vb + (info["tc_pack_floats"] * 4 if precision == 32 else 0)
+        # what FactorBatch.bytes() reports once both directions have run: factors and stencils,
+        # factorization scratch, a slot's 74 vectors and its tagged sweep results (value and tag;
+        # one FP32 set with several slots also keeps them interleaved)
+        results = 2 * (info["update_len"] + 2 * sym.N) * vb
         self.bytes = (self.n_species * N_BINS * (info["factor_elems"] * vb + 7 * sym.N * 8)
                       + min(48 << 30, self.n_species * N_BINS * scratch)
-                      + slots * 60 * sym.N * 8)
+                      + slots * (74 * sym.N * 8 + results * (2 if self.n_species == 1 and vb == 4 else 1)))
 
     def build(self):
         """Assemble and factor every species of the entry (on the caller's stream)."""

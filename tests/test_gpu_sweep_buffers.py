@@ -105,3 +105,23 @@ def test_first_sweeps_of_two_handles_at_once(bits):
     ref.numeric(T, d)
     for a, trans in zip(out[0], (True, False)):
         assert torch.equal(ref.chain(x, trans=trans, refine=False), a)
+
+
+@pytest.mark.parametrize("bits,species,slots", [(32, 3, 8), (32, 1, 8), (64, 2, 3)])
+def test_a_served_entry_is_admitted_by_what_it_comes_to_hold(bits, species, slots):
+    import torch
+    from orbit_b200 import synthetic
+    from orbit_b200.serve import _Entry
+    from orbit_b200.symbolic import Symbolic
+    shape = (6, 10, 12)
+    mets = synthetic.make_met(5, *shape, cmfmc_frac=0.3)
+    e = _Entry(None, Symbolic(*shape), mets, [synthetic.make_species(6 + q, *shape).sink_diag(mets) for q in range(species)],
+               slots, bits)
+    e.build()
+    x = torch.exp(torch.randn(slots, e.sym.N, dtype=torch.float64, device="cuda"))
+    for n in (1, slots):
+        for trans in (False, True):
+            e.fb.chain(x[:n], trans=trans, refine=False)
+    held = sum(e.fb.bytes())
+    e.release()
+    assert held <= e.bytes <= 1.01 * held
