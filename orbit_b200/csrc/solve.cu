@@ -374,36 +374,25 @@ __device__ __forceinline__ int group_lanes(int maxlen) {
     }                                                                       \
   } while (0)
 
-// Column-oriented partial dot products of the transposed sweeps: this warp's
-// share (rows i0 + warp, i0 + warp + kWarps, ... below i1) of
-// sum_i a[i * stride] v_k[i] for nk <= K vectors v_k = v + k * vcap, with
-// four loads in flight (lanes hold consecutive columns, so every row step is
-// one coalesced 128-byte read per warp).
-template <typename T, int K>
-__device__ __forceinline__ void col_dot(const T* __restrict__ a, int64_t stride, int i0, int i1, const T* v,
-                                        int vcap, int nk, T (&acc)[K]) {
+// Column-oriented partial dot product of the transposed sweeps with whole-subtree
+// tasks: this warp's share (rows i0 + warp, i0 + warp + kWarps, ... below i1) of
+// sum_i a[i * stride] v[i], added to acc, with four loads in flight (lanes hold
+// consecutive columns, so every row step is one coalesced read per warp).
+template <typename T>
+__device__ __forceinline__ T col_dot(const T* __restrict__ a, int64_t stride, int i0, int i1, const T* v, T acc) {
   int i = i0 + (threadIdx.x >> 5);
   for (; i + 3 * kWarps < i1; i += 4 * kWarps) {
     const T x0 = __ldg(a + (int64_t)i * stride);
     const T x1 = __ldg(a + (int64_t)(i + kWarps) * stride);
     const T x2 = __ldg(a + (int64_t)(i + 2 * kWarps) * stride);
     const T x3 = __ldg(a + (int64_t)(i + 3 * kWarps) * stride);
-#pragma unroll
-    for (int k = 0; k < K; ++k)
-      if (k < nk) {
-        const T* vk = v + k * vcap;
-        acc[k] = fma(x0, vk[i], acc[k]);
-        acc[k] = fma(x1, vk[i + kWarps], acc[k]);
-        acc[k] = fma(x2, vk[i + 2 * kWarps], acc[k]);
-        acc[k] = fma(x3, vk[i + 3 * kWarps], acc[k]);
-      }
+    acc = fma(x0, v[i], acc);
+    acc = fma(x1, v[i + kWarps], acc);
+    acc = fma(x2, v[i + 2 * kWarps], acc);
+    acc = fma(x3, v[i + 3 * kWarps], acc);
   }
-  for (; i < i1; i += kWarps) {
-    const T x = __ldg(a + (int64_t)i * stride);
-#pragma unroll
-    for (int k = 0; k < K; ++k)
-      if (k < nk) acc[k] = fma(x, v[k * vcap + i], acc[k]);
-  }
+  for (; i < i1; i += kWarps) acc = fma(__ldg(a + (int64_t)i * stride), v[i], acc);
+  return acc;
 }
 
 // Forward step of one supernode (L, or U^T when trans) for output rows
@@ -472,12 +461,8 @@ __device__ __forceinline__ void fwd_node(const ChainDev<T>& D, int o, int tau, i
     const T* Qr = SQ + (int64_t)(n + m) * ldn;
     for (int cb = r0; cb < r1; cb += 32) {
       const int c = cb + lane;
-      T a1[1] = {T(0)};
-      if (c < r1) {
-        if (c < n) col_dot<T, 1>(SQ + c, ldn, 0, c + 1, vec, 0, 1, a1);
-        else col_dot<T, 1>(Qr + (c - n), ldm, 0, n, vec, 0, 1, a1);
-      }
-      const T acc = a1[0];
+      T acc = T(0);
+      if (c < r1) acc = c < n ? col_dot(SQ + c, ldn, 0, c + 1, vec, acc) : col_dot(Qr + (c - n), ldm, 0, n, vec, acc);
       red[warp * 32 + lane] = acc;
       __syncthreads();
       if (warp == 0 && c < r1) {
@@ -530,12 +515,8 @@ __device__ __forceinline__ void bwd_node(const ChainDev<T>& D, int o, int tau, i
     const T* Pb = SQ + (int64_t)n * ldn;
     for (int cb = r0; cb < r1; cb += 32) {
       const int c = cb + lane;
-      T a1[1] = {T(0)};
-      if (c < r1) {
-        col_dot<T, 1>(SQ + c, ldn, c + 1, n, vec, 0, 1, a1);
-        col_dot<T, 1>(Pb + c, ldn, 0, m, vec + n0pad, 0, 1, a1);
-      }
-      const T acc = a1[0];
+      T acc = T(0);
+      if (c < r1) acc = col_dot(Pb + c, ldn, 0, m, vec + n0pad, col_dot(SQ + c, ldn, c + 1, n, vec, acc));
       red[warp * 32 + lane] = acc;
       __syncthreads();
       if (warp == 0 && c < r1) {
@@ -995,59 +976,63 @@ __device__ __forceinline__ bool flow_gather_bwd(const ChainDev<T>& D, int o, int
       });
 }
 
-// Column sums of the transposed sweeps: for the columns [c0, c1) of a
-// row-major block (16-byte aligned at column c0, at most LPR vectors wide),
-// sum over rows [i0, i1) of a[i][c] v[i], terms outside the triangle dropped
-// (TRI 1: i <= c, 2: i > c; c counted from the block's first column).  LPR
-// lanes hold one row's vectors, so the block's 128 threads read 4 * 32 / LPR
-// rows per step with U 16-byte loads in flight per lane, where one column per
-// lane would have four 4-byte ones.  Partial sums over a lane's rows.
-template <typename T, int LPR, int TRI, int U>
-__device__ __forceinline__ void col_part(const T* __restrict__ a, int64_t ld, int c0, int i0, int i1, const T* v,
-                                         uint64_t pol, T (&acc)[Vec16<T>::w]) {
-  using V = typename Vec16<T>::type;
-  constexpr int W = Vec16<T>::w, RW = 32 / LPR, STEP = kWarps * RW;
-  const int lane = threadIdx.x & 31, cl = lane % LPR;
-  const int c = c0 + cl * W;
-  const T* base = a + c;
-  for (int i = i0 + (threadIdx.x >> 5) * RW + lane / LPR; i < i1; i += U * STEP) {
-    V x[U];
+// Column sums of the transposed FP64 sweeps.  A column's sum is sixteen chains of
+// fused multiply-adds, chain p over the rows congruent to p mod 16 of its block
+// (U^T: SQ, or Qr; L^T: [SQ; Pb]) in increasing order; chains 4 w .. 4 w + 3 are
+// added in pairs, the four sums of w in order.  The order fixes the rounding
+// whatever the chunk, the lanes per row or the kernel (k_flow_t, k_chain_multi),
+// so that a receptor's result does not depend on the batch that it is solved in.
+constexpr int kColClasses = 16;
+
+// For a row-major block (16-byte aligned at column c0, LPR vectors wide), sum over
+// rows [i0, i1) (i0 a multiple of 16) of a[i][c] v[i], terms outside the triangle
+// left out (TRI 1: i <= c, 2: i > c; c counted from the block's first column).  LPR lanes hold one
+// row's vectors, so the block's 128 threads read 4 * 32 / LPR rows per step with U
+// 16-byte loads in flight per lane, where one column per lane would have four
+// 4-byte ones.  Warp w takes the chains 4 w .. 4 w + 3, LPR / 8 of them per lane.
+template <int LPR, int TRI, int U>
+__device__ __forceinline__ void col_part(const double* __restrict__ a, int64_t ld, int c0, int i0, int i1,
+                                         const double* v, uint64_t pol, double (&acc)[LPR / 8][2]) {
+  constexpr int Q = LPR / 8;
+  const int lane = threadIdx.x & 31;
+  const int c = c0 + (lane % LPR) * 2;
+  const double* base = a + c;
+  for (int i = i0 + (threadIdx.x >> 5) * 4 + lane / LPR * Q; i < i1; i += U / Q * kColClasses) {
+    double2 x[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      x[u] = V{};
-      if (u == 0 || i + u * STEP < i1) x[u] = ld_stream(reinterpret_cast<const V*>(base + (int64_t)(i + u * STEP) * ld), pol);
+      const int r = i + u / Q * kColClasses + u % Q;
+      x[u] = double2{};
+      if (u == 0 || r < i1) x[u] = ld_stream(reinterpret_cast<const double2*>(base + (int64_t)r * ld), pol);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int r = i + u * STEP;
+      const int r = i + u / Q * kColClasses + u % Q;
       if (u == 0 || r < i1) {
-        const T b = v[r];
-        const T* xe = reinterpret_cast<const T*>(&x[u]);
-#pragma unroll
-        for (int k = 0; k < W; ++k) {
-          const bool in = TRI == 0 || (TRI == 1 ? r <= c + k : r > c + k);
-          acc[k] = fma(in ? xe[k] : T(0), b, acc[k]);
-        }
+        const double b = v[r];
+        if (TRI == 0 || (TRI == 1 ? r <= c : r > c)) acc[u % Q][0] = fma(x[u].x, b, acc[u % Q][0]);
+        if (TRI == 0 || (TRI == 1 ? r <= c + 1 : r > c + 1)) acc[u % Q][1] = fma(x[u].y, b, acc[u % Q][1]);
       }
     }
   }
 }
 
-// Sum of the lanes' and warps' column partials; red: kWarps x LPR * W.  The
-// thread c < LPR * W returns column c's sum.  Two block barriers.
-template <typename T, int LPR>
-__device__ __forceinline__ T col_reduce(T (&acc)[Vec16<T>::w], T* red) {
-  constexpr int W = Vec16<T>::w, CB = LPR * W;
+// Sum of the chains; red: kWarps x LPR * 2.  The thread c < LPR * 2 returns column
+// c's sum.  Two block barriers.
+template <int LPR>
+__device__ __forceinline__ double col_reduce(double (&acc)[LPR / 8][2], double* red) {
+  constexpr int CB = LPR * 2;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int k = 0; k < W; ++k)
+  for (int k = 0; k < 2; ++k) {
+    double x = acc[0][k];
+    if constexpr (LPR == 16) x += acc[1][k];
 #pragma unroll
-    for (int o = LPR; o < 32; o <<= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
-  if (lane < LPR)
-#pragma unroll
-    for (int k = 0; k < W; ++k) red[warp * CB + lane * W + k] = acc[k];
+    for (int o = LPR; o < 32; o <<= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    if (lane < LPR) red[warp * CB + lane * 2 + k] = x;
+  }
   __syncthreads();
-  T sum = T(0);
+  double sum = 0.0;
   if (threadIdx.x < CB)
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) sum += red[w * CB + threadIdx.x];
@@ -1169,37 +1154,36 @@ __device__ __forceinline__ void flow_chains(const ChainDev<float>& D, bool fwd, 
   }
 }
 
-// Column blocks [cb, cb + LPR * W) of a transposed FP64 task.
-template <typename T, int LPR>
-__device__ __forceinline__ void flow_cols(const ChainDev<T>& D, bool fwd, int o, int tau, int s, int n, int m,
-                                          int first, int r0, int r1, const T* SQ, const T* vec, T* red,
+// Column blocks [cb, cb + 2 LPR) of a transposed FP64 task (its chunk starts at a
+// multiple of 16 columns of SQ or of Qr).
+template <int LPR>
+__device__ __forceinline__ void flow_cols(const ChainDev<double>& D, bool fwd, int o, int tau, int s, int n, int m,
+                                          int first, int r0, int r1, const double* SQ, const double* vec, double* red,
                                           uint64_t pol) {
-  constexpr int W = Vec16<T>::w, CB = LPR * W, U = sizeof(T) == 4 ? 4 : 6;
+  constexpr int CB = LPR * 2, U = 6;
   const int ldn = D.ldn[s], ldm = D.ldm[s];
   for (int cb = r0; cb < r1; cb += CB) {
-    T acc[W];
-#pragma unroll
-    for (int k = 0; k < W; ++k) acc[k] = T(0);
+    double acc[LPR / 8][2] = {};
     const int cend = min(cb + CB, r1);
     // lanes whose vector starts at or beyond the row's padded end read nothing
     const int cl = (threadIdx.x & 31) % LPR;
     if (fwd) {
       if (cb < n) {  // U^T: rows i <= c
-        if (cb + cl * W < ldn) {
-          col_part<T, LPR, 0, U>(SQ, ldn, cb, 0, cb, vec, pol, acc);
-          col_part<T, LPR, 1, U>(SQ, ldn, cb, cb, min(cend, n), vec, pol, acc);
+        if (cb + cl * 2 < ldn) {
+          col_part<LPR, 0, U>(SQ, ldn, cb, 0, cb, vec, pol, acc);
+          col_part<LPR, 1, U>(SQ, ldn, cb, cb, min(cend, n), vec, pol, acc);
         }
-      } else if (cb - n + cl * W < ldm) {
-        col_part<T, LPR, 0, U>(SQ + (int64_t)(n + m) * ldn, ldm, cb - n, 0, n, vec, pol, acc);
+      } else if (cb - n + cl * 2 < ldm) {
+        col_part<LPR, 0, U>(SQ + (int64_t)(n + m) * ldn, ldm, cb - n, 0, n, vec, pol, acc);
       }
-    } else if (cb + cl * W < ldn) {  // L^T, unit diagonal; [SQ; Pb] is one block of n + m rows
-      col_part<T, LPR, 2, U>(SQ, ldn, cb, cb + 1, min(cb + CB, n), vec, pol, acc);
-      col_part<T, LPR, 0, U>(SQ, ldn, cb, min(cb + CB, n), n + m, vec, pol, acc);
+    } else if (cb + cl * 2 < ldn) {  // L^T, unit diagonal; [SQ; Pb] is one block of n + m rows
+      col_part<LPR, 2, U>(SQ, ldn, cb, cb, min(cb + CB, n + m), vec, pol, acc);
+      col_part<LPR, 0, U>(SQ, ldn, cb, cb + CB, n + m, vec, pol, acc);
     }
-    const T sum = col_reduce<T, LPR>(acc, red);
+    const double sum = col_reduce<LPR>(acc, red);
     const int c = cb + threadIdx.x;
     if (threadIdx.x < CB && c < cend)
-      flow_put_col<T>(D, fwd, o, tau, s, n, first, c, fwd && c >= n ? vec[c] : T(0), fwd ? sum : vec[c] + sum);
+      flow_put_col<double>(D, fwd, o, tau, s, n, first, c, fwd && c >= n ? vec[c] : 0.0, fwd ? sum : vec[c] + sum);
   }
 }
 
@@ -1375,8 +1359,8 @@ __global__ void __launch_bounds__(kSolveThreads, 5)
 // per SM (16 at 8 blocks, 1 / 4 / 12 orbits of the 40x36x15 grid: 1.49 / 1.93 /
 // 2.58 ms; 32: 1.31 / 1.79 / 2.71), 12 in FP64.  Against one column per lane with
 // four loads in flight and a completion counter per supernode: 40x36x15 FP32
-// 1 / 12 orbits 3.25 / 5.03 -> 1.31 / 2.71 ms, FP64 1 orbit 2.38 -> 1.00;
-// 80x72x15 FP32 12 orbits 11.5 -> 9.1, FP64 1 orbit 4.22 -> 1.96.
+// 1 / 12 orbits 3.25 / 5.03 -> 1.31 / 2.71 ms, FP64 1 orbit 2.38 -> 0.92;
+// 80x72x15 FP32 12 orbits 11.5 -> 9.1, FP64 1 orbit 4.22 -> 1.82.
 template <typename T>
 __global__ void __launch_bounds__(kSolveThreads, 7) k_flow_t(ChainDev<T> D) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1423,20 +1407,23 @@ __global__ void __launch_bounds__(kSolveThreads, 7) k_flow_t(ChainDev<T> D) {
       else if (r1 - r0 >= 64) flow_chains<2>(D, fwd, o, tau, s, n, m, first, r0, r1, SQ, vec, red, pol);
       else flow_chains<1>(D, fwd, o, tau, s, n, m, first, r0, r1, SQ, vec, red, pol);
     } else {
-      if (r1 - r0 <= 16) flow_cols<T, 8>(D, fwd, o, tau, s, n, m, first, r0, r1, SQ, vec, red, pol);
-      else flow_cols<T, 16>(D, fwd, o, tau, s, n, m, first, r0, r1, SQ, vec, red, pol);
+      if (r1 - r0 <= 16) flow_cols<8>(D, fwd, o, tau, s, n, m, first, r0, r1, SQ, vec, red, pol);
+      else flow_cols<16>(D, fwd, o, tau, s, n, m, first, r0, r1, SQ, vec, red, pol);
     }
     __syncthreads();  // the record is read until here
   }
 }
 
-// ---- many right-hand sides on one factor set ----
+// ---- many FP64 right-hand sides on one factor set ----
 //
-// When every solve slot of a handle maps onto the same factor set (marginal
+// When every solve slot of an FP64 handle maps onto the same factor set (marginal
 // perturbations or adjoint receptors of one operator), each task serves a
 // group of K right-hand sides: one claim, one dependency wait (on the group's
 // counters) and one barrier sequence, and every factor row loaded once is
-// multiplied against the K gathered vectors.  Non-transposed sweeps only.
+// multiplied against the K gathered vectors.  Transposed sums have the order of
+// k_flow_t's (16 right-hand sides of the 40x36x15 grid, a transposed sweep: 4.68
+// ms with each lane's rows starting at its own column, 3.89 with the warp's rows
+// together).
 
 template <typename T, int G, int K>
 __device__ __forceinline__ void dot_seg_multi(const T* __restrict__ a, const T* v, int vcap, int nk, int j0, int j1,
@@ -1471,6 +1458,33 @@ __device__ __forceinline__ void dot_seg_multi(const T* __restrict__ a, const T* 
     for (int k = 0; k < K; ++k)
       if (k < nk) acc[k] = fma(x, v[k * vcap + j], acc[k]);
   }
+}
+
+// This warp's four chains of a column (see col_part), for K right-hand sides, and
+// their sum: a at row 0 of the column's block, v by its rows.
+template <typename T, int K>
+__device__ __forceinline__ void col_dot_multi(const T* __restrict__ a, int64_t stride, int i0, int i1, const T* v,
+                                              int vcap, int nk, T (&sum)[K]) {
+  T acc[4][K] = {};
+  int i = (i0 & ~(kColClasses - 1)) + (threadIdx.x >> 5) * 4;
+  auto rows = [&](bool ends) {
+    T x[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      x[q] = !ends || (i + q >= i0 && i + q < i1) ? __ldg(a + (int64_t)(i + q) * stride) : T(0);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (!ends || (i + q >= i0 && i + q < i1))
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+          if (k < nk) acc[q][k] = fma(x[q], v[k * vcap + i + q], acc[q][k]);
+    i += kColClasses;
+  };
+  if (i < i0) rows(true);  // no rows of it where i + 4 <= i0
+  while (i + 4 <= i1) rows(false);
+  if (i < i1) rows(true);
+#pragma unroll
+  for (int k = 0; k < K; ++k) sum[k] = (acc[0][k] + acc[1][k]) + (acc[2][k] + acc[3][k]);
 }
 
 template <int G, int K, typename T, typename P, typename S>
@@ -1603,8 +1617,8 @@ __global__ void __launch_bounds__(kSolveThreads, kChainBlocks[sizeof(T) == 8]) k
 #pragma unroll
         for (int k = 0; k < K; ++k) acc[k] = T(0);
         if (c < r1) {
-          if (c < n) col_dot<T, K>(SQ + c, ldn, 0, c + 1, vbuf, vcap, nk, acc);
-          else col_dot<T, K>(Qr + (c - n), ldm, 0, n, vbuf, vcap, nk, acc);
+          if (c < n) col_dot_multi<T, K>(SQ + c, ldn, 0, c + 1, vbuf, vcap, nk, acc);
+          else col_dot_multi<T, K>(Qr + (c - n), ldm, 0, n, vbuf, vcap, nk, acc);
         }
 #pragma unroll
         for (int k = 0; k < K; ++k) red[(k * kWarps + warp) * 32 + lane] = acc[k];
@@ -1630,28 +1644,24 @@ __global__ void __launch_bounds__(kSolveThreads, kChainBlocks[sizeof(T) == 8]) k
         const double* Yo = D.Y + (int64_t)o[k] * D.N;
         const double* Xout = D.X + ((int64_t)o[k] * 9 + tau) * D.N;
         for (int i = r0 + tid; i < n; i += kSolveThreads) vec[i] = (T)Yo[first + i];
-        for (int u = tid; u < m; u += kSolveThreads) vec[n0pad + u] = (T)Xout[ui[u]];
+        for (int u = tid; u < m; u += kSolveThreads) vec[n + u] = (T)Xout[ui[u]];
       }
       __syncthreads();
-      const T* Pb = SQ + (int64_t)n * ldn;
       for (int cb = r0; cb < r1; cb += 32) {
         const int c = cb + lane;
         T acc[K];
 #pragma unroll
         for (int k = 0; k < K; ++k) acc[k] = T(0);
-        if (c < r1) {
-          col_dot<T, K>(SQ + c, ldn, c + 1, n, vbuf, vcap, nk, acc);
-          col_dot<T, K>(Pb + c, ldn, 0, m, vbuf + n0pad, vcap, nk, acc);
-        }
+        if (c < r1) col_dot_multi<T, K>(SQ + c, ldn, c + 1, n + m, vbuf, vcap, nk, acc);
 #pragma unroll
         for (int k = 0; k < K; ++k) red[(k * kWarps + warp) * 32 + lane] = acc[k];
         __syncthreads();
         if (warp == 0 && c < r1) {
           for (int k = 0; k < nk; ++k) {
-            T sum = vbuf[k * vcap + c];
+            T sum = T(0);
 #pragma unroll
             for (int w2 = 0; w2 < kWarps; ++w2) sum += red[(k * kWarps + w2) * 32 + lane];
-            D.X[((int64_t)o[k] * 9 + tau) * D.N + first + c] = (double)sum;
+            D.X[((int64_t)o[k] * 9 + tau) * D.N + first + c] = (double)(vbuf[k * vcap + c] + sum);
           }
         }
         __syncthreads();
