@@ -414,10 +414,13 @@ int fct_source(int nz, int ny, int nx, const orbit_met_t* met, int n_vec, const 
   const int64_t N = (int64_t)nz * ny * nx;
   FctGeom G{*met, nz, ny, nx, dt, ghost};
   const int tiles = ((nx + kFT - 1) / kFT) * ((ny + kFT - 1) / kFT);
+  int dev = 0, sms = 0;
+  ORBIT_CUDA_TRY(cudaGetDevice(&dev));
+  ORBIT_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   // as many vectors per block (sharing its geometry) as leave about eight blocks
   // per SM
   const int64_t blocks = (int64_t)tiles * nz;
-  const int groups = (int)std::max<int64_t>(1, std::min<int64_t>(n_vec, (8 * 148 + blocks - 1) / blocks));
+  const int groups = (int)std::max<int64_t>(1, std::min<int64_t>(n_vec, (8 * sms + blocks - 1) / blocks));
   const int per = (n_vec + groups - 1) / groups;
   k_fct_source<<<dim3((unsigned)blocks, (n_vec + per - 1) / per), kFT * kFT, 0, st>>>(G, c, n_vec, per, limited, d, N);
   note_launch();
