@@ -43,13 +43,23 @@ namespace {
 // Blocks per SM the counter kernels are compiled for, per precision: many hide
 // more of the per-task latency of launches that fill the GPU (FP32 10 with 48
 // registers, FP64 7 with 72), fewer leave registers for the loads in flight of
-// the others.  FP32, 80x72x15 grid, 8 bins, 1 / 4 / 12 orbits at 10 and at 8
-// blocks: 1.55 / 2.74 / 6.03 and 1.39 / 2.62 / 6.25 ms, 60x54x15 with 12 orbits 3.77
-// and 3.41; FP64, 1 / 2 / 4 orbits at 7 and at 6: 1.81 / 2.65 / 4.00 and 1.73 /
-// 2.73 / 4.11, 60x54x15 with 4 orbits 2.47 and 2.35.  So the line lies between the
-// factor bytes of one bin of all orbits in those launches.
+// the others.  Sums do not depend on it.  8 bins, ms, many / few, with the factor
+// entries of one bin of all orbits:
+//   FP32 80x72x15: 1 orbit (52 M) 1.48 / 1.32, 4 (208 M) 2.67 / 2.54, 8 (416 M) 4.36 /
+//   4.19, 10 (520 M) 5.07 / 5.15, 12 5.94 / 6.15; 60x54x15: 4 (105 M) 1.99 / 1.70, 12
+//   (315 M) 3.69 / 3.33, 16 (420 M) 4.35 / 4.24, 24 (631 M) 6.33 / 6.39; 40x36x15: 24
+//   (219 M) 3.05 / 2.75, 48 (439 M) 4.85 / 5.01.
+//   FP64 60x54x15: 2 (53 M) 1.64 / 1.55, 4 (105 M) 2.41 / 2.30, 8 (210 M) 4.41 / 4.08, 12
+//   (315 M) 5.30 / 5.29; 40x36x15: 10 (91 M) 3.40 / 3.10, 24 (219 M) 4.35 / 4.22;
+//   64x60x15: 4 (134 M) 2.88 / 2.74, 6 (201 M) 3.63 / 3.80.  80x72x15, whose tree is
+//   larger: 1 (52 M) 1.75 / 1.67, 2 (104 M) 2.59 / 2.67, 3 3.30 / 3.21, 4 (207 M) 3.94 /
+//   4.06, 6 5.73 / 5.93.
+// So the line lies at 1.6 GB a bin (400 M and 200 M entries) and, for FP64 trees of
+// more than 40 M entries, at 0.6 GB, between one orbit and two.
 constexpr int kChainBlocks[2] = {10, 7}, kChainBlocksFew[2] = {8, 6};  // FP32, FP64
-constexpr double kChainManyBytes[2] = {1.6e9, 0.6e9};
+inline double chain_many_bytes(const Symbolic& S, bool fp64) {
+  return fp64 && S.fac_nnz > 40000000 ? 0.6e9 : 1.6e9;
+}
 constexpr int kSolveThreads = ORBIT_SOLVE_THREADS;
 constexpr int kMaxPhases = 96;  // 2 x tree levels
 constexpr int kWarps = kSolveThreads / 32;
@@ -2642,7 +2652,7 @@ int launch_chain_t(orbit_factor_s* f, double* X, int B, const int* d_orbit_ids, 
       rows ? kStageBytes + sizeof(T) * ((size_t)S.max_front + 8)
            : sizeof(T) * ((size_t)kWarps * 32 * (flow && sizeof(T) == 4 ? 4 : 1) +
                           std::max<size_t>(S.max_front + 8, (size_t)kWarps * ((S.max_sub_front + 7) & ~3)) + 8);
-  const bool few = (double)Bt * S.fac_nnz * sizeof(T) <= kChainManyBytes[sizeof(T) == 8];
+  const bool few = (double)Bt * S.fac_nnz * sizeof(T) <= chain_many_bytes(S, sizeof(T) == 8);
   const void* kfn = rows    ? (const void*)k_flow<T>
                     : flow  ? (const void*)k_flow_t<T>
                     : !sub  ? (few ? (const void*)k_chain<T, false, false, true> : (const void*)k_chain<T, false, false, false>)
