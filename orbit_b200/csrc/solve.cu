@@ -1760,13 +1760,17 @@ __global__ void __launch_bounds__(kSolveThreads, kChainBlocks[sizeof(T) == 8]) k
 // read once is used K times.  Bound by the shared-memory reads of the K vectors
 // (16 bytes per 4 multiply-adds and row): four rows (or two columns) per lane
 // share each of them, and the multiply-adds run two right-hand sides per
-// instruction.  Every right-hand side's sums have the order of the kernels
-// with four of them per task (k_chain_multi), whatever K is.
+// instruction.  A right-hand side's sums have one order whatever K is.  Of a row:
+// G lanes (from its chunk in the schedule of groups of four), each with every Gth
+// vector of four entries, a vector's products added up (second, first, third,
+// fourth) before they join the lane's sum, then a butterfly over the lanes.  Of a
+// column: the four chains of flow_chains.
 //
-// What is left is per-task latency (claim, wait, gather: 6 of a task's 12 us) at
-// two blocks per SM, which the vectors of the largest fronts allow.  80x72x15
-// grid, 8 bins, 64 right-hand sides, a sweep against groups of four with one row
-// (column) per lane: 18.0 -> 8.0 ms, transposed 17.4 -> 9.0 ms.
+// What is left is latency (the wait, the gather and the barriers around them) at
+// two blocks per SM, which the vectors of the largest fronts allow: 41 % of the
+// issue slots used, transposed 33 %.  80x72x15 grid, 8 bins, 64 right-hand sides, a
+// sweep against groups of four with one row (column) per lane: 18.0 -> 8.0 ms,
+// transposed 17.4 -> 9.1 ms.
 constexpr int kMultiThreads = 256;
 constexpr int kMultiWarps = kMultiThreads / 32;
 constexpr size_t kMultiSmem = 108 * 1024;  // two blocks per SM
@@ -2128,7 +2132,7 @@ template <int K, int VEC>
 __device__ __forceinline__ void multi_cols(const MultiDev& M, const FlowRec& R, int gi, const int* o, int nk, int tau,
                                            const float* SQ, float4* V) {
   const ChainDev<float>& D = M.C;
-  constexpr int CB = 32 * VEC, U = 8, QC = K / 4;  // U 4 / 8 / 12 / 16 / 32: 9.3 / 8.2 / 8.4 / 8.7 / 12.5 ms a sweep
+  constexpr int CB = 32 * VEC, U = 8, QC = K / 4;  // U 4 / 8 / 12 / 16: 10.5 / 9.5 / 9.9 / 10.5 ms a sweep of dense vectors
   const bool fwd = R.kind_len == 2;
   const int r0 = R.r0, r1 = R.r1, n = R.n, m = R.m, first = R.first, ldn = R.ldn, ldm = R.ldm;
   const int lane = threadIdx.x & 31, half = threadIdx.x >> 7, w = (threadIdx.x >> 5) & 3, ht = threadIdx.x & 127;
@@ -2256,9 +2260,9 @@ __global__ void __launch_bounds__(kMultiThreads, 2) k_multi(MultiDev M) {
   const int tid = threadIdx.x, lane = tid & 31;
   build_slots(D, s_tab);
   const uint64_t pol = stream_policy(false);
-  // The last warp claims the next task during the gather of the current one (a
-  // claim takes 1.7 us of a task's 12; every dependency is claimed earlier, so the
-  // earliest unfinished task is still the current one of its block).
+  // The last warp claims the next task during the gather of the current one, which
+  // takes the claim's 1.7 us off a task's 12 (every dependency is claimed earlier,
+  // so the earliest unfinished task is still the current one of its block).
   const bool claimer = tid >= kMultiThreads - 32;
   int slot = 0;
   if (claimer) flow_claim(D, s_tab, s_claims[0], slot, K);

@@ -199,8 +199,9 @@ constexpr int kSchedGroups[kNumSched] = {1, 3, 7};
 // Whether a launch of B groups is bound by its dependency chain rather than by
 // the factor values it reads: up to 40 M factor entries per bin of all groups,
 // 60 M where a group's tree is small (its chunks are few).  k_flow against
-// k_chain, 8 bins, ms: 24x20x15 FP64 1 orbit 0.45 / 0.96, FP32 24 orbits (52 M) 1.54
-// / 1.76; 40x36x15 FP64 4 orbits (37 M) 1.65 / 1.74, FP32 4 1.09 / 1.41; 53x47x13
+// k_chain, 8 bins, ms: 24x20x15 FP64 1 orbit 0.45 / 0.96, 28 (60 M) 2.58 / 2.80, FP32 24
+// (52 M) 1.47 / 1.71, 28 (60 M) 1.70 / 1.78, 32 (69 M) 1.94 / 1.83; 30x26x12 FP32 20 orbits
+// (59 M) 1.66 / 1.77, FP64 16 (47 M) 2.05 / 2.53; 40x36x15 FP64 4 orbits (37 M) 1.65 / 1.74, FP32 4 1.09 / 1.41; 53x47x13
 // FP64 2 orbits (30 M) 1.32 / 1.40, FP32 4 (59 M) 1.64 / 1.56; 60x54x15 FP64 1 orbit
 // (26 M) 1.27 / 1.35, FP32 2 (53 M) 1.68 / 1.32; 80x72x15 FP64 1 orbit (52 M) 2.4 /
 // 1.7.
