@@ -369,9 +369,9 @@ int orbit_factor_numeric(orbit_factor_t f, int n_active, const double* const* T_
  * t_factor/t_solve wall times per species (orbit/core/orbit.py:331-383). */
 int orbit_factor_profile(orbit_factor_t f, int mode, double* out);
 /* Device bytes held by the factor handle (reference: numeric_bytes, solve.py:233-236).
- * The workspace grows by up to two buffers, 2 (update entries + 2 N) factor
- * values per slot each, when a sweep that keeps its results there first runs
- * (ORBIT_ERR_NOMEM where the device has no room for them). */
+ * The workspace of an FP32 handle with several slots on one set grows by 2
+ * (update entries + 2 N) factor values per slot when one slot is first swept
+ * alone (ORBIT_ERR_NOMEM where the device has no room for them). */
 int orbit_factor_bytes(orbit_factor_t f, int64_t* numeric_bytes, int64_t* workspace_bytes);
 
 /* K4: chained solves x <- P_tau x for tau in [tau0, tau1) (trans = 0), or

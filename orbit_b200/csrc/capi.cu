@@ -192,17 +192,26 @@ int flow_table(orbit_symbolic_s* sy, FlowKind kind, int k, cudaStream_t st, cons
   return ORBIT_OK;
 }
 
-int sweep_buffers(orbit_factor_s* f, bool multi) {
+// FP32 handles of several slots on one factor set sweep them together.
+static bool sweeps_together(const orbit_factor_s* f) {
+  return f->precision == ORBIT_PREC_FP32 && f->n_sets == 1 && f->n_orbits > 1;
+}
+
+// Bytes of the tagged results of all slots (value and tag), or of the interleaved
+// ones (whole groups of 16, 8 or 4: fewer than twice the slots).
+static size_t sweep_bytes(const orbit_factor_s* f) {
   const Symbolic& S = f->sym->S;
-  const size_t bytes = 2 * (size_t)f->n_orbits * (S.w_size + 2 * S.N) * (f->precision == ORBIT_PREC_FP32 ? 4 : 8);
-  if (multi && !f->multi) {
-    // whole groups of 16, 8 or 4: fewer than twice the orbits
-    ORBIT_TRY(dalloc(f->allocs, reinterpret_cast<unsigned char**>(&f->multi), bytes));
-    f->multi_bytes = bytes;
-  } else if (!multi && !f->flow) {
-    ORBIT_TRY(dalloc(f->allocs, &f->flow, bytes));  // value and tag
-    f->flow_bytes = bytes;
-  }
+  return 2 * (size_t)f->n_orbits * (S.w_size + 2 * S.N) * (f->precision == ORBIT_PREC_FP32 ? 4 : 8);
+}
+
+int sweep_buffers(orbit_factor_s* f, bool multi) {
+  if (multi ? f->multi != nullptr : f->flow != nullptr) return ORBIT_OK;
+  const size_t bytes = sweep_bytes(f);
+  unsigned char* p = nullptr;
+  ORBIT_TRY(dalloc(f->allocs, &p, bytes));
+  f->sweep_bytes += bytes;
+  if (multi) f->multi = reinterpret_cast<float*>(p);
+  else f->flow = p;
   return ORBIT_OK;
 }
 
@@ -575,7 +584,19 @@ int orbit_factor_create_ex(orbit_symbolic_t sym, int n_orbits, int n_sets, int n
   if ((rc = dalloc(A, &f->A_stencil, (size_t)n_inst * 7 * N))) return fail(rc);
   if ((rc = dalloc(A, &f->d_Tptr, (size_t)n_inst))) return fail(rc);
   if ((rc = dalloc(A, &f->d_Dptr, (size_t)n_inst))) return fail(rc);
-  if ((rc = dalloc(A, &f->X, (size_t)n_orbits * 9 * N))) return fail(rc);
+  {
+    // The chain vectors and, in the same allocation (one of their own took 0.2 to
+    // 1 ms, during the first sweep or here), the sweeps' results: interleaved
+    // where slots are swept together, else tagged.
+    const size_t xb = ((size_t)n_orbits * 9 * N * sizeof(double) + 255) / 256 * 256;
+    const size_t rb = S.max_sub_front == 0 ? sweep_bytes(f) : 0;
+    unsigned char* p = nullptr;
+    if ((rc = dalloc(A, &p, xb + rb))) return fail(rc);
+    f->X = reinterpret_cast<double*>(p);
+    f->sweep_bytes = rb;
+    if (rb > 0 && sweeps_together(f)) f->multi = reinterpret_cast<float*>(p + xb);
+    else if (rb > 0) f->flow = p + xb;
+  }
   if ((rc = dalloc(A, &f->Ybuf, (size_t)n_orbits * N))) return fail(rc);
   if ((rc = dalloc(A, &f->Wbuf, (size_t)n_orbits * S.w_size))) return fail(rc);
   if ((rc = dalloc(A, &f->counters, (size_t)n_orbits * 16 * S.nsuper))) return fail(rc);
@@ -604,8 +625,8 @@ int orbit_factor_create_ex(orbit_symbolic_t sym, int n_orbits, int n_sets, int n
     return fail(ORBIT_ERR_NOMEM);
   }
   if (cudaMemset(f->status, 0, sizeof(int)) != cudaSuccess) return fail(ORBIT_ERR_CUDA);
-  // what the forward sweeps of all slots take; the other sweeps' is made when
-  // they first run
+  // the schedule that the forward sweeps of all slots take; the others' are made
+  // when they first run
   if ((rc = prepare_sweeps(f, n_orbits, 0, nullptr))) return fail(rc);
   *out = f;
   return ORBIT_OK;
@@ -700,8 +721,7 @@ int orbit_factor_bytes(orbit_factor_t f, int64_t* numeric_bytes, int64_t* worksp
     *workspace_bytes = (int64_t)2 * f->front_group * S.front_buf_size * vb +
                        (f->tc_pack ? (int64_t)f->front_group * S.tc_pack_size * 4 : 0) +
                        (int64_t)f->n_sets * f->n_bins * 7 * S.N * 8 +
-                       (int64_t)f->n_orbits * (9 + 1 + 8 + 23 + 33) * S.N * 8 + (int64_t)f->flow_bytes +
-                       (int64_t)f->multi_bytes;
+                       (int64_t)f->n_orbits * (9 + 1 + 8 + 23 + 33) * S.N * 8 + (int64_t)f->sweep_bytes;
   return ORBIT_OK;
 }
 

@@ -76,13 +76,13 @@ struct orbit_factor_s {
   double* Wbuf = nullptr;   // w_size
   int* counters = nullptr;  // 8 * 2 * nsuper
   // tagged results of the dataflow chain kernels, all orbits: w_size update
-  // entries, N forward results and N solutions each; made when a launch first
-  // takes those kernels
+  // entries, N forward results and N solutions each
   unsigned char* flow = nullptr;
-  size_t flow_bytes = 0;
-  // interleaved results of the FP32 many-right-hand-side kernels, likewise
+  // interleaved results of the FP32 many-right-hand-side kernels.  A handle is
+  // made with one of the two, behind X; FP32 handles with several slots on one
+  // set make the tagged ones when a single slot is first swept.
   float* multi = nullptr;
-  size_t multi_bytes = 0;
+  size_t sweep_bytes = 0;   // of both
   unsigned flow_seq = 0x0fffffffu;  // launches (28 bits), the tags' high part; the first starts over
   double* E = nullptr;      // 8 N forcing (new order)
   double* tmpv = nullptr;   // 4 N scratch vectors
@@ -112,7 +112,7 @@ struct orbit_factor_s {
 namespace orbit {
 // Device table of one dataflow schedule (the arguments of build_flow).
 int flow_table(orbit_symbolic_s* sy, FlowKind kind, int k, cudaStream_t st, const DevSym::Flow** out);
-// The handle's tagged (multi: interleaved) buffers.
+// The handle's tagged (multi: interleaved) results, made where it has none yet.
 int sweep_buffers(orbit_factor_s* f, bool multi);
 // What the sweeps of B slots need beside the handle's own: both of the above.
 int prepare_sweeps(orbit_factor_s* f, int B, int trans, cudaStream_t st);

@@ -2638,7 +2638,7 @@ int launch_chain_t(orbit_factor_s* f, double* X, int B, const int* d_orbit_ids, 
     // starts over, the first launch being one of those
     unsigned seq = (f->flow_seq + 1) & 0x0fffffffu;
     if (seq == 0) {
-      ORBIT_CUDA_TRY(cudaMemsetAsync(f->flow, 0, f->flow_bytes, st));
+      ORBIT_CUDA_TRY(cudaMemsetAsync(f->flow, 0, 2 * sizeof(T) * (size_t)f->n_orbits * (S.w_size + 2 * S.N), st));
       seq = 1;
     }
     f->flow_seq = seq;

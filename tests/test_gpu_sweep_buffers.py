@@ -1,8 +1,8 @@
 """What the dataflow sweeps keep beside a factor handle (B200).
 
-A handle is made with what the forward sweeps of all its slots take; the
-schedules and buffers of other sweeps are made, cleared on the launch's stream
-and counted when a launch first takes them.
+A handle is made with the tagged results, or where its slots are swept together
+with the interleaved ones; schedules, and the tagged results of the latter
+handles, are made by the launch that first takes them, and counted from then on.
 """
 import threading
 
@@ -52,25 +52,25 @@ def test_made_by_the_launches_that_take_them():
     assert torch.equal(own.chain(x[:1], trans=True, refine=False), one)
 
 
-def test_large_batches_hold_none_until_transposed():
+@pytest.mark.parametrize("bits,slots,sets", [(64, 3, 3), (64, 3, 1), (32, 3, 3), (32, 1, 1), (32, 2, 5)])
+def test_other_handles_do_not_grow(bits, slots, sets):
     import torch
     from orbit_b200 import device
     from orbit_b200.symbolic import Symbolic
-    shape = (15, 54, 60)
+    shape = (6, 10, 12)
     sym = Symbolic(*shape)
-    assert 2 * sym.lunz > 40e6  # two slots' forward sweep is not bound by its chain
-    fixed = device.FactorBatch(sym, 1, 32, n_sets=2)  # one slot's is
-    two = device.FactorBatch(sym, 2, 32)
-    per_slot = 8 * 74 * sym.N
-    assert two.bytes()[1] + _tagged(sym, 1, 32) == fixed.bytes()[1] + per_slot
-    T, d = _inputs(shape, 2)
-    two.numeric(T, d)
-    x = torch.exp(torch.randn(2, sym.N, dtype=torch.float64, device="cuda"))
-    before = two.bytes()[1]
-    two.chain(x, refine=False)
-    assert two.bytes()[1] == before
-    two.chain(x, trans=True, refine=False)
-    assert two.bytes()[1] == before + _tagged(sym, 2, 32)
+    T, d = _inputs(shape, sets)
+    fb = device.FactorBatch(sym, slots, bits, n_sets=sets)
+    more = device.FactorBatch(sym, slots + 1, bits, n_sets=sets)
+    made = fb.bytes()[1]
+    if slots > 1:
+        assert more.bytes()[1] - made == 8 * 74 * sym.N + _tagged(sym, 1, bits)
+    fb.numeric(T, d)
+    x = torch.exp(torch.randn(slots, sym.N, dtype=torch.float64, device="cuda"))
+    for n in (1, slots):
+        for trans in (False, True):
+            assert torch.isfinite(fb.chain(x[:n], trans=trans, refine=False)).all()
+    assert fb.bytes()[1] == made
 
 
 @pytest.mark.parametrize("bits", [32, 64])
